@@ -31,6 +31,17 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// Matrix descriptor of an MN-major tile with one K row (C = 16 or 32 bfloat16
+// channels, 32 or 64 bytes) per line, swizzled over that line as TMA writes it
+// (layout 6 = 32 B, 4 = 64 B): 8 K rows form an atom, the next 8 follow at SBO;
+// the next C M (or N) elements lie `lbo` bytes on. The tile starts on a
+// multiple of 1024 bytes and `saddr` on a multiple of 8 lines.
+template <int C>
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, uint32_t lbo) {
+    static_assert(C == 16 || C == 32, "one atom per line");
+    return smem_desc(saddr, lbo, (uint32_t)(8 * C * 2)) | ((uint64_t)(C == 32 ? 4 : 6) << 61);
+}
+
 // Instruction descriptor of kind::f16 with bfloat16 A and B and a binary32
 // accumulator: D format at bits 4-5 (1 = f32), A and B formats at bits 7-9
 // and 10-12 (1 = bf16), A and B major at bits 15 and 16 (1 = MN-major),

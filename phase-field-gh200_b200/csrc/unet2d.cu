@@ -316,7 +316,12 @@ struct pfb_sur2d {
             (rc = alloc(&dphi, B * kImg * kImg)) || (rc = alloc(&origins, B * 2)) ||
             (rc = alloc(&loss_partial, (size_t)kLossBlocks)))
             return rc;
+        // partial sums of the weight gradients: one block per SM, also for
+        // batches of a few crops
+        int sms = 0;
+        SUR_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
         wg_bytes = conv3x3_wgrad_workspace(mb, kImg, kImg, 32, 32);
+        if (const size_t all = (size_t)sms * (9 * 32 * 32 + 32) * sizeof(float); wg_bytes < all) wg_bytes = all;
         if ((rc = alloc(&wg_ws, wg_bytes / sizeof(float)))) return rc;
         // He-normal weights on the real input channels; the last layer starts
         // at zero (identity jump), padded channels stay zero
