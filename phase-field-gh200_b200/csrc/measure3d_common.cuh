@@ -58,6 +58,10 @@ __device__ __forceinline__ void load_row6(const T* plane, int B, int y, int x0, 
 
 // Sums of one item: columns x0 .. x0 + 3 of rows y0 .. y0 + 3 of brick plane
 // z (world plane wz); pm, pc, pp are planes z - 1, z, z + 1.
+//
+// Bound by the instructions a voxel takes: whether a row of four holds
+// anything non-finite, supported or large enough to carry own quanta is told
+// by its largest |phi| bit pattern, and only such rows pay for it.
 template <typename T = float>
 __device__ __forceinline__ void measure_item(const MeasureCell& M, const T* pm,
                                              const T* pc, const T* pp, int x0, int y0,
@@ -72,13 +76,16 @@ __device__ __forceinline__ void measure_item(const MeasureCell& M, const T* pm,
 #pragma unroll
     for (int j = 0; j < 4; ++j) wxj[j] = wrap_offset(M.ox, x0 + j, L.nx);
     // aggregate words of a row, fetched one row ahead
-    auto load_agg = [&](int y, uint32_t* out) {
-        const size_t srow = s_index(L, 0, wrap_offset(M.oy, y, L.ny), wz);
+    const uint32_t* splane = M.S + s_index(L, 0, 0, wz);
+    int wy = wrap_offset(M.oy, y0, L.ny);
+    auto load_agg = [&](uint32_t* out) {
+        const uint32_t* row = splane + (size_t)wy * (size_t)L.pitch_x;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) out[j] = __ldg(M.S + srow + wxj[j]);
+        for (int j = 0; j < 4; ++j) out[j] = __ldg(row + wxj[j]);
+        wy = wy + 1 < L.ny ? wy + 1 : 0;
     };
     uint32_t agg_next[4];
-    load_agg(y0, agg_next);
+    load_agg(agg_next);
 #pragma unroll 1
     for (int r = 0; r < 4; ++r) {
         const int y = y0 + r;
@@ -89,41 +96,63 @@ __device__ __forceinline__ void measure_item(const MeasureCell& M, const T* pm,
         uint32_t agg[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) agg[j] = agg_next[j];
-        if (r < 3) load_agg(y + 1, agg_next);
+        if (r < 3) load_agg(agg_next);
+        uint32_t m = max4(rc + 1);
+        float cz[4] = {rc[1], rc[2], rc[3], rc[4]};  // a non-finite sample counts as 0
+        bool fin[4] = {true, true, true, true};
+        if (m >= kInfBits) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                fin[j] = isfinite(cz[j]);
+                if (!fin[j]) {
+                    ++cnt.nonfinite;
+                    cz[j] = 0.0f;
+                }
+            }
+            m = max4(cz);
+        }
+        if (m > kQZeroBits) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t own = q_of3(cz[j]);
+                const bool neg = agg[j] < own;
+                cnt.negative += neg ? 1u : 0u;
+                agg[j] = neg ? 0u : agg[j] - own;
+            }
+        }
         double rV = 0.0, rX = 0.0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float c = rc[j + 1];
-            const bool cfin = isfinite(c);
-            cnt.nonfinite += cfin ? 0u : 1u;
+            const float c = cz[j];
             const float gx = 0.5f * (rc[j + 2] - rc[j]);
             const float gy = 0.5f * (rn[j + 1] - rs[j + 1]);
             const float gz = 0.5f * (zpv[j] - zmv[j]);
-            const uint32_t own = q_of3(c);
-            const bool nz = cfin && c != 0.0f;
-            const bool neg = nz && agg[j] < own;
-            cnt.negative += neg ? 1u : 0u;
-            float other = (nz && !neg) ? (float)(agg[j] - own) * kQInv : 0.0f;
+            // where c is 0 the product is 0 whatever the aggregate holds
+            float other = (float)agg[j] * kQInv;
             if (M.wall) other += wallv;
-            const double sq = cfin ? (double)c * (double)c : 0.0;
+            const double sq = (double)c * (double)c;
             rV += sq;
-            rX += sq * (double)j;
-            if (M.surface && cfin)
+            if (j == 1) rX = sq;
+            if (j > 1) rX += sq * (double)j;
+            if (M.surface && fin[j])
                 acc.Sf += sqrt((double)gx * gx + (double)gy * gy + (double)gz * gz);
-            acc.Ix += cfin ? (double)(c * gx * other) : 0.0;
-            acc.Iy += cfin ? (double)(c * gy * other) : 0.0;
-            acc.Iz += cfin ? (double)(c * gz * other) : 0.0;
-            if (cfin) acc.pmax = max(acc.pmax, __float_as_uint(fabsf(c)));
-            const int x = x0 + j;
-            if (cfin && fabsf(c) > kSupportEps3) {
-                if (top_plane) ++cnt.top;
-                acc.lox = min(acc.lox, x);
-                acc.hix = max(acc.hix, x);
-                acc.loy = min(acc.loy, y);
-                acc.hiy = max(acc.hiy, y);
-                acc.loz = min(acc.loz, z);
-                acc.hiz = max(acc.hiz, z);
-            }
+            const float fx = c * gx * other, fy = c * gy * other, fz = c * gz * other;
+            acc.Ix += fin[j] ? (double)fx : 0.0;
+            acc.Iy += fin[j] ? (double)fy : 0.0;
+            acc.Iz += fin[j] ? (double)fz : 0.0;
+        }
+        acc.pmax = max(acc.pmax, m);
+        if (m > __float_as_uint(kSupportEps3)) {
+            unsigned mask = 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) mask |= fabsf(cz[j]) > kSupportEps3 ? 1u << j : 0u;
+            if (top_plane) cnt.top += __popc(mask);
+            acc.lox = min(acc.lox, x0 + __ffs(mask) - 1);
+            acc.hix = max(acc.hix, x0 + 31 - __clz(mask));
+            acc.loy = min(acc.loy, y);
+            acc.hiy = max(acc.hiy, y);
+            acc.loz = min(acc.loz, z);
+            acc.hiz = max(acc.hiz, z);
         }
         acc.V += rV;
         acc.Cx += rV * (double)x0 + rX;

@@ -66,5 +66,14 @@ __device__ __forceinline__ void phi_st4(T* o, const float* v, const uint16_t* b)
     }
 }
 
+// |phi| up to here squares to less than half a quantum: q_of3 gives 0.
+constexpr uint32_t kQZeroBits = 0x387BA882u;  // 6.0e-5f
+constexpr uint32_t kInfBits = 0x7F800000u;
+
+__device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7FFFFFFFu; }
+__device__ __forceinline__ uint32_t max4(const float* v) {
+    return max(max(abs_bits(v[0]), abs_bits(v[1])), max(abs_bits(v[2]), abs_bits(v[3])));
+}
+
 }  // namespace p3
 }  // namespace pfb
