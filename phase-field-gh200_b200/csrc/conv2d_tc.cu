@@ -68,6 +68,7 @@ struct ConvFwdArgs {
     const bf16* x;     // [B][P2][CIN]
     bf16* y;           // [B][P2][COUT] or null
     float* yf;         // [B][P2][COUT] or null (binary32 copy of the output)
+    float* y0;         // [B][H W] or null (channel 0 of the output, no border)
     const bf16* w;     // packed [9][CIN / 8][COUT][8]
     const float* bias; // [COUT] or null
     const bf16* gate;  // [B][P2][COUT] or null: output *= (gate > 0)
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3_fwd(const __grid_const
                     *reinterpret_cast<float4*>(A.yf + o + 4 * h) =
                         make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
             }
+            if (A.y0 && interior) A.y0[((size_t)b * A.H + (q / W2 - 1)) * A.W + (xp - 1)] = acc[0];
             }
         }
     }
@@ -212,37 +214,50 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3_fwd(const __grid_const
 // ---- forward, persistent and warp-specialised ----------------------------------
 // The same contraction as k_conv3x3_fwd with the three stages of a tile in
 // separate warps so that they overlap across tiles: warp 0 loads a tile's
-// chunk planes with TMA (cp.async.bulk.tensor, a 4D view of the activations:
-// 8 channels x channel chunk x position x image, so positions outside the
-// image arrive as zeros) into a two-stage ring; warp 1 issues the tile's
-// tcgen05 MMAs into one of two TMEM accumulators and commits; warps 2-5
-// (one TMEM lane quadrant each) run the epilogue of the previous tile. The
-// packed weights are staged once per CTA with one bulk copy. Each CTA walks
-// tiles c, c + G, c + 2G, ... of the B x tiles work list.
-constexpr int kWsThreads = 192;
+// positions with TMA (cp.async.bulk.tensor, channels x positions x images, so
+// positions outside the image arrive as zeros; a position's channels are one
+// row of 64 or 32 bytes, swizzled over that width) into a ring of stages; warp
+// 1 issues the tile's tcgen05 MMAs into one of two TMEM accumulators and
+// commits; eight epilogue warps (one TMEM lane quadrant of one M-tile each) drain
+// the previous tile. One staged copy serves all nine taps: a tap only moves the
+// descriptor's first row, and the swizzle, which works on shared-memory
+// address bits, stays in step with what TMA wrote. The packed weights are
+// staged once per CTA with one bulk copy. Each CTA walks tiles c, c + G,
+// c + 2G, ... of the B x tiles work list.
+//
+// Bound by the number of MMAs (45 clocks each up to N = 64, 36 a tile) and the
+// activations' DRAM traffic (143 MB, 22 us): 256 crops of 64 x 64, 32 -> 32
+// channels take 45 us (55 us gated) against 74 (84) of one tile per CTA.
+// Side-by-side taps (N = 96, a third of the MMAs, neighbouring lanes added by
+// shuffles) measured 128 us with one CTA per SM, where this form took 53.
+constexpr int kWsThreads = 64 + 128 * kConvMT;  // producer, MMA, epilogue warps of each M-tile
 constexpr int kWsStages = 2;
+constexpr int kWsHeader = 1024;  // barriers, bias
 
-// rows per TMA box: half the staged rows, rounded up to 8 (two boxes per plane)
+// rows per TMA box: half the staged rows, rounded up to 8 (two boxes)
 __host__ __device__ constexpr int ws_box(int W) { return round_up((fwd_rows(W) + 1) / 2, 8); }
-__host__ __device__ constexpr int ws_plane(int W) { return round_up(2 * ws_box(W) * 16, 128); }
+template <int CIN>
+__host__ __device__ constexpr int ws_stage(int W) { return round_up(2 * ws_box(W) * CIN * 2, 1024); }
 
 template <int CIN, int COUT>
 __host__ __device__ constexpr int ws_smem(int W) {
-    return 1024 + kWsStages * (CIN / 8) * ws_plane(W) + 9 * (CIN / 8) * COUT * 16;
+    return kWsHeader + kWsStages * ws_stage<CIN>(W) + 9 * CIN * COUT * 2;
 }
 
 struct WsHeader {
     uint64_t full[kWsStages], empty[kWsStages], acc_full[2], acc_empty[2], wbar;
     uint32_t tmem_slot;
     int fail;
+    alignas(16) float bias[64];
 };
+static_assert(sizeof(WsHeader) <= kWsHeader, "header");
 
-__device__ __forceinline__ void tma_load4(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                          int c3, uint32_t bar) {
+__device__ __forceinline__ void tma_load3(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
+                                          uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
         : "memory");
 }
 
@@ -257,21 +272,22 @@ __global__ void __launch_bounds__(kWsThreads)
     WsHeader& H = *reinterpret_cast<WsHeader*>(smem);
     const int W2 = A.W + 2;
     const int P2 = (A.H + 2) * W2;
-    const int CH = ws_plane(A.W);
     const int BOX = ws_box(A.W);
-    unsigned char* sA = smem + 1024;                                // stages x planes
-    unsigned char* sW = sA + (size_t)kWsStages * NCA * CH;          // packed weights
+    const int STAGE = ws_stage<CIN>(A.W);
+    constexpr int ROW = CIN * 2;  // bytes of a position
+    unsigned char* sA = smem + kWsHeader;                // stages
+    unsigned char* sW = sA + (size_t)kWsStages * STAGE;  // packed weights
     const uint32_t sa = dev::smem_addr(sA), sw = dev::smem_addr(sW);
-    const uint32_t stage_bytes = (uint32_t)(NCA * 2 * BOX * 16);
+    const uint32_t stage_bytes = (uint32_t)(2 * BOX * ROW);
     const uint32_t wbytes = (uint32_t)(9 * NCA * COUT * 16);
 
     const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int items = A.B * A.tiles;
     const int q_end = (A.H + 1) * W2;
 
-    // every TMA destination below is 128-byte aligned when the dynamic
-    // shared memory is; refuse to run otherwise
-    if (dev::smem_addr(smem) & 127u) {
+    // the swizzle works on address bits: stages start on multiples of 1024
+    // bytes when the dynamic shared memory does; refuse to run otherwise
+    if (dev::smem_addr(smem) & 1023u) {
         if (tid == 0) atomicOr(&g_conv_status, 2u);
         return;
     }
@@ -282,7 +298,7 @@ __global__ void __launch_bounds__(kWsThreads)
         }
         for (int a = 0; a < 2; ++a) {
             dev::mbar_init(&H.acc_full[a], 1);
-            dev::mbar_init(&H.acc_empty[a], 4);  // one arrival per epilogue warp
+            dev::mbar_init(&H.acc_empty[a], 4 * kConvMT);  // one arrival per epilogue warp
         }
         dev::mbar_init(&H.wbar, 1);
         H.fail = 0;
@@ -294,6 +310,7 @@ __global__ void __launch_bounds__(kWsThreads)
         tc::tmem_alloc(&H.tmem_slot, NCOLS);
         tc::tmem_relinquish();
     }
+    if (tid >= 64 && tid < 64 + COUT) H.bias[tid - 64] = A.bias ? A.bias[tid - 64] : 0.0f;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -304,7 +321,7 @@ __global__ void __launch_bounds__(kWsThreads)
     };
 
     if (warp == 0 && lane == 0) {
-        // ---- producer: chunk planes of each tile, two boxes per plane
+        // ---- producer: the positions of each tile, two boxes
         int k = 0;
         for (int it = (int)blockIdx.x; it < items && !H.fail; it += (int)gridDim.x, ++k) {
             const int s = k % kWsStages;
@@ -316,10 +333,8 @@ __global__ void __launch_bounds__(kWsThreads)
             const int qa = t * (kConvMT * 128) - 1;  // first staged position (W2 + t 256 - (W2 + 1))
             const uint32_t bar = dev::smem_addr(&H.full[s]);
             dev::mbar_arrive_expect_tx(&H.full[s], stage_bytes);
-            for (int c = 0; c < NCA; ++c)
-                for (int h = 0; h < 2; ++h)
-                    tma_load4(sa + (uint32_t)((s * NCA + c) * CH + h * BOX * 16), &X, 0, c, qa + h * BOX, b,
-                              bar);
+            for (int h = 0; h < 2; ++h)
+                tma_load3(sa + (uint32_t)(s * STAGE + h * BOX * ROW), &X, 0, qa + h * BOX, b, bar);
         }
         // no copy may still target shared memory at exit
         for (int j = (k > kWsStages ? k - kWsStages : 0); j < k; ++j)
@@ -329,6 +344,7 @@ __global__ void __launch_bounds__(kWsThreads)
         // ---- MMA issue
         if (!dev::mbar_wait_bounded(&H.wbar, 0, tc::kMmaWaitPolls)) give_up();
         constexpr uint32_t idesc = tc::idesc_bf16_f32(128, COUT, false, false);
+        const uint64_t w0 = tc::smem_desc(sw, (uint32_t)(COUT * 16), 128u);
         int k = 0;
         for (int it = (int)blockIdx.x; it < items && !H.fail; it += (int)gridDim.x, ++k) {
             const int s = k % kWsStages, a = k & 1;
@@ -338,20 +354,24 @@ __global__ void __launch_bounds__(kWsThreads)
                 break;
             }
             tc::fence_after_sync();
-            const uint32_t st = sa + (uint32_t)(s * NCA * CH);
-            for (int m = 0; m < kConvMT; ++m)
-                for (int tap = 0; tap < 9; ++tap) {
-                    const int dy = tap / 3, dx = tap - 3 * (tap / 3);
-                    const int row = m * 128 + dy * W2 + dx;
-                    for (int ks = 0; ks < CIN / 16; ++ks) {
-                        const uint64_t ad =
-                            tc::smem_desc(st + (uint32_t)(2 * ks * CH + row * 16), (uint32_t)CH, 128u);
-                        const uint64_t bd = tc::smem_desc(sw + (uint32_t)((tap * NCA + 2 * ks) * COUT * 16),
-                                                          (uint32_t)(COUT * 16), 128u);
-                        tc::mma_bf16(tmem + (uint32_t)(a * ACC + m * COUT), ad, bd, idesc,
-                                     (tap | ks) ? 1u : 0u);
-                    }
+            const uint32_t st = sa + (uint32_t)(s * STAGE);
+            // start-address fields advance by bytes / 16
+            const uint64_t a0 = tc::smem_desc_k<CIN>(st);
+#pragma unroll
+            for (int m = 0; m < kConvMT; ++m) {
+                const uint32_t d = tmem + (uint32_t)(a * ACC + m * COUT);
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy) {
+                    const uint64_t ay = a0 + (uint64_t)(uint32_t)((m * 128 + dy * W2) * (ROW / 16));
+#pragma unroll
+                    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+                        for (int ks = 0; ks < CIN / 16; ++ks)
+                            tc::mma_bf16(d, ay + (uint64_t)(dx * (ROW / 16) + 2 * ks),
+                                         w0 + (uint64_t)(((3 * dy + dx) * NCA + 2 * ks) * COUT), idesc,
+                                         (dy | dx | ks) ? 1u : 0u);
                 }
+            }
             tc::mma_commit(&H.empty[s]);     // the stage may be refilled
             tc::mma_commit(&H.acc_full[a]);  // the accumulator may be read
         }
@@ -360,73 +380,75 @@ __global__ void __launch_bounds__(kWsThreads)
             (void)dev::mbar_wait_bounded(&H.acc_full[(k - 1) & 1], (uint32_t)(((k - 1) >> 1) & 1),
                                          tc::kMmaWaitPolls);
     } else if (warp >= 2) {
-        // ---- epilogue: TMEM lane quadrant warp % 4
-        const int quad = warp & 3;
-        const int r = quad * 32 + lane;
+        // ---- epilogue: TMEM lane quadrant warp % 4 of M-tile (warp - 2) / 4
+        const int quad = warp & 3, m = (warp - 2) >> 2;
+        const int r = m * 128 + quad * 32 + lane;
         int k = 0;
         for (int it = (int)blockIdx.x; it < items; it += (int)gridDim.x, ++k) {
             const int a = k & 1;
+            const int b = it / A.tiles, t = it - b * A.tiles;
+            const int q = W2 + t * (kConvMT * 128) + r;
+            const bool in = q < q_end;
+            const int xp = q % W2;
+            const bool interior = xp >= 1 && xp <= A.W;
+            const size_t o = ((size_t)b * P2 + q) * COUT;
+            // the gate arrives while the tile's MMAs run
+            uint4 gv[COUT / 8];
+            const bool gated = A.gate && in && interior;
+            if (gated)
+#pragma unroll
+                for (int h = 0; h < COUT / 8; ++h)
+                    gv[h] = __ldg(reinterpret_cast<const uint4*>(A.gate + o) + h);
             const bool ok = dev::mbar_wait_bounded(&H.acc_full[a], (uint32_t)((k >> 1) & 1), tc::kMmaWaitPolls);
             if (!__all_sync(0xFFFFFFFFu, ok) || H.fail) {
                 if (lane == 0 && !ok) give_up();
                 break;
             }
             tc::fence_after_sync();
-            const int b = it / A.tiles, t = it - b * A.tiles;
-            const int q0 = W2 + t * (kConvMT * 128);
-            for (int m = 0; m < kConvMT; ++m) {
-                float acc[COUT];
+#pragma unroll
+            for (int h = 0; h < COUT / 16; ++h) {
                 __syncwarp();  // the TMEM loads are warp-collective
+                uint32_t u[16];
+                tc::tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * ACC + m * COUT + 16 * h), u);
+                tc::tmem_wait_ld();
+                if (!in) continue;
+                float v[16];
 #pragma unroll
-                for (int h = 0; h < COUT / 16; ++h) {
-                    uint32_t v[16];
-                    tc::tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * ACC + m * COUT + 16 * h), v);
-                    tc::tmem_wait_ld();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[16 * h + j] = __uint_as_float(v[j]);
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 bj = *reinterpret_cast<const float4*>(&H.bias[16 * h + j]);
+                    v[j] = __uint_as_float(u[j]) + bj.x;
+                    v[j + 1] = __uint_as_float(u[j + 1]) + bj.y;
+                    v[j + 2] = __uint_as_float(u[j + 2]) + bj.z;
+                    v[j + 3] = __uint_as_float(u[j + 3]) + bj.w;
                 }
-                const int q = q0 + m * 128 + r;
-                if (q >= q_end) continue;
-                const int xp = q % W2;
-                const bool interior = xp >= 1 && xp <= A.W;
-                const size_t o = ((size_t)b * P2 + q) * COUT;
-                float g[COUT];
+                if (A.relu)
 #pragma unroll
-                for (int j = 0; j < COUT; ++j) g[j] = 1.0f;
-                if (A.gate && interior) {
+                    for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
+                if (gated)
 #pragma unroll
-                    for (int h = 0; h < COUT / 8; ++h) {
-                        const uint4 gv = *reinterpret_cast<const uint4*>(A.gate + o + 8 * h);
-                        const bf16* ge = reinterpret_cast<const bf16*>(&gv);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) g[8 * h + j] = __bfloat162float(ge[j]) > 0.0f ? 1.0f : 0.0f;
+                    for (int j = 0; j < 16; ++j) {
+                        const bf16* ge = reinterpret_cast<const bf16*>(&gv[2 * h + j / 8]);
+                        v[j] *= __bfloat162float(ge[j % 8]) > 0.0f ? 1.0f : 0.0f;
                     }
-                }
+                if (!interior)
 #pragma unroll
-                for (int j = 0; j < COUT; ++j) {
-                    float v = acc[j];
-                    if (A.bias) v += A.bias[j];
-                    if (A.relu) v = fmaxf(v, 0.0f);
-                    v *= g[j];
-                    acc[j] = interior ? v : 0.0f;
-                }
-                if (A.y) {
+                    for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+                if (A.y)
 #pragma unroll
-                    for (int h = 0; h < COUT / 8; ++h) {
+                    for (int k8 = 0; k8 < 2; ++k8) {
                         uint4 pk;
                         __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            p2[j] = __floats2bfloat162_rn(acc[8 * h + 2 * j], acc[8 * h + 2 * j + 1]);
-                        *reinterpret_cast<uint4*>(A.y + o + 8 * h) = pk;
+                            p2[j] = __floats2bfloat162_rn(v[8 * k8 + 2 * j], v[8 * k8 + 2 * j + 1]);
+                        *reinterpret_cast<uint4*>(A.y + o + 16 * h + 8 * k8) = pk;
                     }
-                }
-                if (A.yf) {
+                if (A.yf)
 #pragma unroll
-                    for (int h = 0; h < COUT / 4; ++h)
-                        *reinterpret_cast<float4*>(A.yf + o + 4 * h) =
-                            make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
-                }
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<float4*>(A.yf + o + 16 * h + j) =
+                            make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                if (A.y0 && h == 0 && interior) A.y0[((size_t)b * A.H + (q / W2 - 1)) * A.W + (xp - 1)] = v[0];
             }
             // the accumulator is free again
             tc::fence_before_sync();
@@ -443,37 +465,36 @@ __global__ void __launch_bounds__(kWsThreads)
 // dW[tap] = sum over positions p of dY[p - dx] x[p + dy (W + 2)]: both
 // operands are MN-major tiles of kWgKT positions, channels innermost, exactly
 // as TMA lays an activation box down (rows of one position, 64 or 32 bytes,
-// swizzled over that width). A holds three copies of the dY tile shifted by
-// dx = -1, 0, 1 (M = 3 CY of 128 rows; the copies are 16-byte-unit TMA
-// coordinates, not thread work), B the x tile of one dy, so a tile of
-// positions takes 3 MMAs per 16 positions instead of 9 taps' worth of staged
-// columns. The middle row's B operand has a second atom of ones: its column
-// is the bias gradient.
+// swizzled over that width). The 128 rows of A are 128 / CY slots of CY
+// channels, slot s the dY tile moved by s - 1 positions: one staged copy with
+// a leading offset of one row (slots past the third are not used). B holds the
+// x tiles of the three dy and a tile of ones side by side (N = 3 CX + 16: the last columns are the bias gradient),
+// so 16 positions take one MMA. The width matters: a 128-row MMA of K = 16
+// takes 45 clocks up to N = 64 and 58 at N = 112 (measured), so three of N = 32
+// or nine of one tap each would be bound by their number.
 //
 // Warp-specialised and persistent, one CTA per SM: CTA c owns a contiguous
 // range of the B x chunks tiles and accumulates all of it in TMEM; warp 0
 // keeps a ring of kWgStages tiles in flight, warp 1 issues, warps 2-5 write
-// the CTA's partial sums at the end. What bounds it: operand reads of the
-// MMAs (4 KB of A per 32-column MMA) and the TMA fill of 6 tiles per chunk,
-// both from shared memory's 128 B per clock. 256 crops of 64 x 64, 32 -> 32
-// channels: 68 us a layer (training step 2.488 -> 1.688 ms against one CTA per
-// half image that staged nine shifted copies of x with cp.async).
-constexpr int kWgStages = 5;
+// the CTA's partial sums at the end. 256 crops of 64 x 64, 32 -> 32
+// channels: 52 us a layer with the reduction, against about 200 of one CTA per
+// half image that staged nine shifted copies of x with cp.async; bound by the
+// TMA fill (392 rows per tile, 1.3 GB a layer through the L2).
+constexpr int kWgStages = 6;
 constexpr int kWgThreads = 192;
 constexpr int kWgKT = 96;        // positions per tile: divides 64 x 66 exactly
 constexpr int kWgHeader = 1024;  // barriers
-constexpr int kWgOnes = 1024;    // the atom of ones
-constexpr uint32_t kWgCols = 128;  // TMEM: middle row at 0, rows -1 and +1 at 64 and 96
+constexpr uint32_t kWgCols = 128;  // TMEM: CX columns per dy, then 16 of the bias
 
-// A stage holds the 6 tiles, and at least the 128 rows an A operand spans (rows
-// past the 3 tiles are read, their products are not used).
+constexpr int kWgYRows = kWgKT + 8;  // dY rows staged: the last slot is moved by 7 at most
+// A stage: the dY tile, three x tiles, a tile of ones.
+template <int CY>
+__host__ __device__ constexpr int wg_dy_bytes() { return round_up(kWgYRows * CY * 2, 1024); }
 template <int CX, int CY>
-__host__ __device__ constexpr int wg_stage_bytes() {
-    return 3 * (CX + CY) > 128 ? 3 * kWgKT * 2 * (CX + CY) : 128 * kWgKT * 2;
-}
+__host__ __device__ constexpr int wg_stage_bytes() { return wg_dy_bytes<CY>() + 4 * kWgKT * CX * 2; }
 template <int CX, int CY>
 __host__ __device__ constexpr int wg_smem() {
-    return kWgHeader + kWgStages * wg_stage_bytes<CX, CY>() + kWgOnes;
+    return kWgHeader + kWgStages * wg_stage_bytes<CX, CY>();
 }
 
 struct WgHeader {
@@ -489,15 +510,6 @@ struct ConvWgradArgs {
     int items;       // tiles of the batch
 };
 
-__device__ __forceinline__ void tma_load3(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                          uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-        : "memory");
-}
-
 // DY covers image rows 1 .. H of the gradient (positions outside read as
 // zeros), X the whole padded image.
 template <int CX, int CY>
@@ -505,15 +517,14 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     k_conv3x3_wgrad(const __grid_constant__ ConvWgradArgs A, const __grid_constant__ CUtensorMap X,
                     const __grid_constant__ CUtensorMap DY) {
     static_assert((CX == 16 || CX == 32) && (CY == 16 || CY == 32), "one swizzle atom per position");
-    constexpr int AT = kWgKT * CY * 2, BT = kWgKT * CX * 2;  // bytes of an operand tile
+    constexpr int AT = wg_dy_bytes<CY>(), BT = kWgKT * CX * 2;  // bytes of the dY and of an x tile
     constexpr int STAGE = wg_stage_bytes<CX, CY>();
     static_assert(AT % 1024 == 0 && BT % 1024 == 0 && kWgKT % 16 == 0, "tiles keep the swizzle phase");
-    static_assert((128 / CY) * AT <= STAGE, "A rows stay inside the stage");
+    static_assert(kWgKT + 128 / CY - 1 <= kWgYRows, "every slot's rows are staged");
     extern __shared__ __align__(1024) unsigned char smem[];
     WgHeader& H = *reinterpret_cast<WgHeader*>(smem);
     const uint32_t base = dev::smem_addr(smem);
     const uint32_t st0 = base + kWgHeader;
-    const uint32_t ones = st0 + kWgStages * STAGE;
     const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = (int)gridDim.x, c = (int)blockIdx.x;
     const int i0 = (int)((long long)A.items * c / G), i1 = (int)((long long)A.items * (c + 1) / G);
@@ -529,9 +540,11 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         H.fail = aligned ? 0 : 1;
         if (!aligned) atomicOr(&g_conv_status, 2u);
     }
-    if (tid < kWgOnes / 16)
-        *reinterpret_cast<uint4*>(smem + kWgHeader + kWgStages * STAGE + tid * 16) =
+    for (int i = tid; i < kWgStages * (BT / 16); i += kWgThreads) {
+        const int s = i / (BT / 16), j = i - s * (BT / 16);
+        *reinterpret_cast<uint4*>(smem + kWgHeader + s * STAGE + AT + 3 * BT + j * 16) =
             make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+    }
     if (warp == 0) {
         tc::tmem_alloc(&H.tmem_slot, kWgCols);
         tc::tmem_relinquish();
@@ -559,10 +572,10 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             const int b = it / A.chunks, p = (it - b * A.chunks) * kWgKT;
             const uint32_t bar = dev::smem_addr(&H.full[s]);
             const uint32_t st = st0 + (uint32_t)(s * STAGE);
-            dev::mbar_arrive_expect_tx(&H.full[s], (uint32_t)(3 * (AT + BT)));
-            for (int d = 0; d < 3; ++d) tma_load3(st + (uint32_t)(d * AT), &DY, 0, p + 1 - d, b, bar);
+            dev::mbar_arrive_expect_tx(&H.full[s], (uint32_t)(kWgYRows * CY * 2 + 3 * BT));
+            tma_load3(st, &DY, 0, p - 1, b, bar);
             for (int d = 0; d < 3; ++d)
-                tma_load3(st + (uint32_t)(3 * AT + d * BT), &X, 0, p + d * A.W2, b, bar);
+                tma_load3(st + (uint32_t)(AT + d * BT), &X, 0, p + d * A.W2, b, bar);
         }
         // no copy may still target shared memory at exit
         for (int j = (k > kWgStages ? k - kWgStages : 0); j < k; ++j)
@@ -570,8 +583,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                                          tc::kMmaWaitPolls);
     } else if (warp == 1 && lane == 0) {
         // ---- MMA issue
-        constexpr uint32_t id = tc::idesc_bf16_f32(128, CX, true, true);
-        constexpr uint32_t id_mid = tc::idesc_bf16_f32(128, CX + 16, true, true);
+        constexpr uint32_t id = tc::idesc_bf16_f32(128, 3 * CX + 16, true, true);
         constexpr uint32_t KS_A = 16 * CY * 2, KS_B = 16 * CX * 2;  // 16 positions
         int k = 0;
         for (int it = i0; it < i1 && !failed(); ++it, ++k) {
@@ -582,20 +594,19 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             }
             tc::fence_after_sync();
             const uint32_t st = st0 + (uint32_t)(s * STAGE);
+            // a step adds its bytes / 16 to the start-address fields
+            const uint64_t ad0 = tc::smem_desc_mn<CY>(st, (uint32_t)(CY * 2));
+            const uint64_t bd0 = tc::smem_desc_mn<CX>(st + AT, (uint32_t)BT);
 #pragma unroll
-            for (int kk = 0; kk < kWgKT / 16; ++kk) {
-                const uint64_t ad = tc::smem_desc_mn<CY>(st + kk * KS_A, (uint32_t)AT);
-                const uint32_t b0 = st + 3 * AT + kk * KS_B;
-                const uint32_t acc = (k | kk) ? 1u : 0u;
-                tc::mma_bf16(tmem + 64u, ad, tc::smem_desc_mn<CX>(b0, (uint32_t)BT), id, acc);
-                tc::mma_bf16(tmem, ad, tc::smem_desc_mn<CX>(b0 + BT, ones - (b0 + BT)), id_mid, acc);
-                tc::mma_bf16(tmem + 96u, ad, tc::smem_desc_mn<CX>(b0 + 2 * BT, (uint32_t)BT), id, acc);
-            }
+            for (int kk = 0; kk < kWgKT / 16; ++kk)
+                tc::mma_bf16(tmem, ad0 + (uint64_t)(kk * KS_A >> 4), bd0 + (uint64_t)(kk * KS_B >> 4), id,
+                             (k | kk) ? 1u : 0u);
             tc::mma_commit(&H.empty[s]);
         }
         tc::mma_commit(&H.done);
     } else if (warp >= 2) {
-        // ---- partial sums: row slot * CY + co of the accumulator is tap column slot
+        // ---- partial sums: row slot * CY + co of the accumulator is tap column
+        // dx = 1 - slot (dY moved by slot - 1 meets x at the opposite offset)
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const int slot = row / CY, co = row % CY;
@@ -612,14 +623,14 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                const uint32_t col = d == 1 ? 0u : d == 0 ? 64u : 96u;
+                const uint32_t col = (uint32_t)(d * CX);
 #pragma unroll
                 for (int h = 0; h < CX / 16; ++h) {
                     uint32_t v[16];
                     tc::tmem_ld16(lanes + col + (uint32_t)(16 * h), v);
                     tc::tmem_wait_ld();
                     if (slot < 3) {
-                        float* o = out + ((3 * d + slot) * CY + co) * CX + 16 * h;
+                        float* o = out + ((3 * d + 2 - slot) * CY + co) * CX + 16 * h;
                         if (vec) {
 #pragma unroll
                             for (int j = 0; j < 16; j += 4)
@@ -632,7 +643,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                 }
                 if (d == 1) {
                     uint32_t v[16];
-                    tc::tmem_ld16(lanes + (uint32_t)CX, v);
+                    tc::tmem_ld16(lanes + (uint32_t)(3 * CX), v);
                     tc::tmem_wait_ld();
                     if (slot == 1) out[9 * CY * CX + co] = __uint_as_float(v[0]);
                 }
@@ -696,8 +707,15 @@ void launch_wgrad_reduce(const float* partial, int grid, int cx, int cy, float* 
 // Packed weights from OIHW binary32 W[co][ci][3][3] (cout x cin):
 //   forward  : P[tap][ci / 8][co][ci % 8] = W[co][ci][tap]
 //   transpose: P[tap][co / 8][ci][co % 8] = W[co][ci][8 - tap]  (data gradient)
-__global__ void k_pack_weights(const float* __restrict__ w, bf16* __restrict__ p, int cin, int cout,
-                               int transpose) {
+struct PackJobs {
+    ConvPackJob job[16];
+};
+
+__global__ void k_pack_weights(const __grid_constant__ PackJobs J) {
+    const ConvPackJob& job = J.job[blockIdx.y];
+    const float* __restrict__ w = job.w;
+    bf16* __restrict__ p = static_cast<bf16*>(job.packed);
+    const int cin = job.cin, cout = job.cout, transpose = job.transpose;
     const int n = 9 * cin * cout;
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
@@ -731,9 +749,8 @@ cudaError_t launch_fwd(const ConvFwdArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// 0: one tile per CTA; 1: the persistent warp-specialised forward for the
-// 32 -> 32 channel layers (the pairs where it measured faster on a B200);
-// 2: the persistent forward for every built pair. Both honour the width limit.
+// 0: one tile per CTA; 1 and 2: the persistent warp-specialised forward for
+// every built pair where two TMA boxes hold a tile's rows (W <= 124).
 int g_conv_pipeline = 1;
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
@@ -749,6 +766,21 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
     return fn;
 }
 
+// Activations [B][P2][C] (positions pos0 .. pos0 + npos of each image) as a
+// C channels x positions x images map of boxes of `box` positions, swizzled
+// over the C channels of a position.
+bool position_map(CUtensorMap* map, const bf16* base, int C, int P2, int pos0, int npos, int B, int box) {
+    const cuuint64_t dims[3] = {(cuuint64_t)C, (cuuint64_t)npos, (cuuint64_t)B};
+    const cuuint64_t strides[2] = {(cuuint64_t)C * 2, (cuuint64_t)P2 * C * 2};
+    const cuuint32_t boxd[3] = {(cuuint32_t)C, (cuuint32_t)box, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+                          const_cast<bf16*>(base + (size_t)pos0 * C), dims, strides, boxd, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // The persistent forward; *used = false (nothing launched) when the shape or
 // the driver does not allow it.
 template <int CIN, int COUT>
@@ -756,53 +788,39 @@ cudaError_t launch_fwd_ws(const ConvFwdArgs& a, cudaStream_t s, bool* used) {
     *used = false;
     const int smem = ws_smem<CIN, COUT>(a.W);
     PFN_cuTensorMapEncodeTiled_v12000 encode = encode_tiled();
-    if (!g_conv_pipeline || (g_conv_pipeline == 1 && !(CIN == 32 && COUT == 32)) || !encode ||
+    if (!g_conv_pipeline || !encode ||
         ws_box(a.W) > 256 || smem > 227 * 1024)
         return cudaSuccess;
     const int P2 = (a.H + 2) * (a.W + 2);
-    // activations [B][P2][CIN] as 8 channels x CIN/8 chunks x P2 positions x B images
-    const cuuint64_t dims[4] = {8, (cuuint64_t)(CIN / 8), (cuuint64_t)P2, (cuuint64_t)a.B};
-    const cuuint64_t strides[3] = {16, (cuuint64_t)CIN * 2, (cuuint64_t)P2 * CIN * 2};
-    const cuuint32_t box[4] = {8, 1, (cuuint32_t)ws_box(a.W), 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
     CUtensorMap map;
-    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(a.x), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaSuccess;
+    if (!position_map(&map, a.x, CIN, P2, 0, P2, a.B, ws_box(a.W))) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(k_conv3x3_fwd_ws<CIN, COUT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_conv3x3_fwd_ws<CIN, COUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 100);
     if (e != cudaSuccess) return e;
-    int per = 0, dev = 0, sms = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_conv3x3_fwd_ws<CIN, COUT>, kWsThreads,
-                                                           smem)) != cudaSuccess ||
+    int dev = 0, sms = 0;
+    cudaFuncAttributes fa;
+    if ((e = cudaFuncGetAttributes(&fa, k_conv3x3_fwd_ws<CIN, COUT>)) != cudaSuccess ||
         (e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    // every resident CTA must get its TMEM columns (512 per SM)
-    const int cols = 2 * (int)fwd_tmem_cols<COUT>();
-    per = per < 512 / cols ? per : 512 / cols;
-    if (per < 1) return cudaSuccess;
+    // CTAs an SM holds by shared memory (1 KB of it reserved per CTA),
+    // registers and TMEM columns. The runtime's occupancy query is not used:
+    // it answers 1 for this kernel, and one CTA leaves the SM waiting on its
+    // own epilogue.
+    const int by_smem = 228 * 1024 / (smem + 1024);
+    const int by_regs = 65536 / (round_up(fa.numRegs * 32, 256) * (kWsThreads / 32));
+    const int by_tmem = 512 / (2 * (int)fwd_tmem_cols<COUT>());
+    int per = by_smem < by_regs ? by_smem : by_regs;
+    per = per < by_tmem ? per : by_tmem;
+    if (per < 1) per = 1;
     const int items = a.B * a.tiles;
     const int grid = items < sms * per ? items : sms * per;
     k_conv3x3_fwd_ws<CIN, COUT><<<grid, kWsThreads, smem, s>>>(a, map);
     *used = true;
     return cudaGetLastError();
-}
-
-// Activations [B][P2][C] (positions pos0 .. pos0 + npos of each image) as a
-// C channels x positions x images map of kWgKT-position boxes, swizzled over
-// the C channels of a position.
-bool wgrad_map(CUtensorMap* map, const bf16* base, int C, int P2, int pos0, int npos, int B) {
-    const cuuint64_t dims[3] = {(cuuint64_t)C, (cuuint64_t)npos, (cuuint64_t)B};
-    const cuuint64_t strides[2] = {(cuuint64_t)C * 2, (cuuint64_t)P2 * C * 2};
-    const cuuint32_t box[3] = {(cuuint32_t)C, (cuuint32_t)kWgKT, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
-                          const_cast<bf16*>(base + (size_t)pos0 * C), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int CX, int CY>
@@ -811,7 +829,8 @@ cudaError_t launch_wgrad(const ConvWgradArgs& a, const bf16* x, const bf16* dy, 
     constexpr int smem = wg_smem<CX, CY>();
     const int W2 = W + 2, P2 = (H + 2) * W2;
     CUtensorMap mx, my;
-    if (!encode_tiled() || !wgrad_map(&mx, x, CX, P2, 0, P2, B) || !wgrad_map(&my, dy, CY, P2, W2, H * W2, B))
+    if (!encode_tiled() || !position_map(&mx, x, CX, P2, 0, P2, B, kWgKT) ||
+        !position_map(&my, dy, CY, P2, W2, H * W2, B, kWgYRows))
         return cudaErrorNotSupported;
     cudaError_t e = cudaFuncSetAttribute(k_conv3x3_wgrad<CX, CY>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -830,8 +849,8 @@ bool shape_ok(int B, int H, int W) {
 
 int conv3x3_fwd(const void* x, void* y, float* yf, const void* wp, const float* bias,
                 const void* gate, int B, int H, int W, int cin, int cout, int relu,
-                cudaStream_t s) {
-    if (!x || !wp || (!y && !yf)) return set_error(PFB_E_ARG, "conv3x3: null buffer");
+                cudaStream_t s, float* y0) {
+    if (!x || !wp || (!y && !yf && !y0)) return set_error(PFB_E_ARG, "conv3x3: null buffer");
     if (!shape_ok(B, H, W)) return set_error(PFB_E_ARG, "conv3x3: bad shape %dx%dx%d", B, H, W);
     if ((uintptr_t)x % 16 || (uintptr_t)wp % 16 || (y && (uintptr_t)y % 16) ||
         (yf && (uintptr_t)yf % 16) || (gate && (uintptr_t)gate % 16))
@@ -840,6 +859,7 @@ int conv3x3_fwd(const void* x, void* y, float* yf, const void* wp, const float* 
     a.x = static_cast<const bf16*>(x);
     a.y = static_cast<bf16*>(y);
     a.yf = yf;
+    a.y0 = y0;
     a.w = static_cast<const bf16*>(wp);
     a.bias = bias;
     a.gate = static_cast<const bf16*>(gate);
@@ -915,16 +935,27 @@ int conv3x3_wgrad(const void* x, const void* dy, float* workspace, size_t worksp
     return PFB_OK;
 }
 
-int conv3x3_pack(const float* w, void* packed, int cin, int cout, int transpose, cudaStream_t s) {
-    if (!w || !packed) return set_error(PFB_E_ARG, "conv3x3_pack: null buffer");
-    if (cin % 8 || cout % 8 || cin <= 0 || cout <= 0)
-        return set_error(PFB_E_ARG, "conv3x3_pack: channels must be multiples of 8");
-    const int n = 9 * cin * cout;
-    k_pack_weights<<<(n + 255) / 256, 256, 0, s>>>(w, static_cast<bf16*>(packed), cin, cout,
-                                                    transpose ? 1 : 0);
+int conv3x3_pack_many(const ConvPackJob* jobs, int n, cudaStream_t s) {
+    PackJobs J;
+    if (!jobs || n < 1 || n > 16) return set_error(PFB_E_ARG, "conv3x3_pack: bad job list");
+    int most = 0;
+    for (int k = 0; k < n; ++k) {
+        const ConvPackJob& j = jobs[k];
+        if (!j.w || !j.packed) return set_error(PFB_E_ARG, "conv3x3_pack: null buffer");
+        if (j.cin % 8 || j.cout % 8 || j.cin <= 0 || j.cout <= 0)
+            return set_error(PFB_E_ARG, "conv3x3_pack: channels must be multiples of 8");
+        J.job[k] = j;
+        most = most > 9 * j.cin * j.cout ? most : 9 * j.cin * j.cout;
+    }
+    k_pack_weights<<<dim3((unsigned)((most + 255) / 256), (unsigned)n), 256, 0, s>>>(J);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(PFB_E_CUDA, "conv3x3_pack: %s", cudaGetErrorString(e));
     return PFB_OK;
+}
+
+int conv3x3_pack(const float* w, void* packed, int cin, int cout, int transpose, cudaStream_t s) {
+    const ConvPackJob job{w, packed, cin, cout, transpose ? 1 : 0};
+    return conv3x3_pack_many(&job, 1, s);
 }
 
 int conv_read_status(unsigned* out, int clear) {

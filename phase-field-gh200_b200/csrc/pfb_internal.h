@@ -164,10 +164,17 @@ int relax_insert(pfb_sim2d* s, const int* origins, const float* dphi);
 // conv2d_tc.cu: 3x3 same convolutions on padded-NHWC bfloat16 activations
 int conv3x3_fwd(const void* x, void* y, float* yf, const void* wp, const float* bias,
                 const void* gate, int B, int H, int W, int cin, int cout, int relu,
-                cudaStream_t s);
+                cudaStream_t s, float* y0 = nullptr);
 size_t conv3x3_wgrad_workspace(int B, int H, int W, int cx, int cy);
 int conv3x3_wgrad(const void* x, const void* dy, float* workspace, size_t workspace_bytes,
                   float* dw, float* db, int B, int H, int W, int cx, int cy, cudaStream_t s);
+// One packing of conv3x3_pack; conv3x3_pack_many runs up to 16 in one launch.
+struct ConvPackJob {
+    const float* w;
+    void* packed;
+    int cin, cout, transpose;
+};
+int conv3x3_pack_many(const ConvPackJob* jobs, int n, cudaStream_t s);
 int conv3x3_pack(const float* w, void* packed, int cin, int cout, int transpose, cudaStream_t s);
 int conv_read_status(unsigned* out, int clear);
 

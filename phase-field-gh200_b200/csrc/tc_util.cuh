@@ -35,11 +35,23 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
 // channels, 32 or 64 bytes) per line, swizzled over that line as TMA writes it
 // (layout 6 = 32 B, 4 = 64 B): 8 K rows form an atom, the next 8 follow at SBO;
 // the next C M (or N) elements lie `lbo` bytes on. The tile starts on a
-// multiple of 1024 bytes and `saddr` on a multiple of 8 lines.
+// multiple of 1024 bytes; the swizzle works on address bits, so neither `saddr`
+// nor `lbo` need be a multiple of an atom (lbo = one line: the next C elements
+// are the same channels one K row on).
 template <int C>
 __device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, uint32_t lbo) {
     static_assert(C == 16 || C == 32, "one atom per line");
     return smem_desc(saddr, lbo, (uint32_t)(8 * C * 2)) | ((uint64_t)(C == 32 ? 4 : 6) << 61);
+}
+
+// Matrix descriptor of a K-major tile whose rows are C = 16 or 32 bfloat16
+// channels (32 or 64 bytes), swizzled over that row as TMA writes it; `saddr`
+// is the first row plus 32 bytes per K = 16 step, and the row need not start
+// an 8-row atom.
+template <int C>
+__device__ __forceinline__ uint64_t smem_desc_k(uint32_t saddr) {
+    static_assert(C == 16 || C == 32, "one swizzle span per row");
+    return smem_desc(saddr, 16u, (uint32_t)(8 * C * 2)) | ((uint64_t)(C == 32 ? 4 : 6) << 61);
 }
 
 // Instruction descriptor of kind::f16 with bfloat16 A and B and a binary32

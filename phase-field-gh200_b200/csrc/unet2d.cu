@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kEwThreads) k_loss(const float* __restrict__ o
     for (int t = (int)(blockIdx.x * blockDim.x + threadIdx.x); t < n; t += gridDim.x * blockDim.x) {
         const int b = t / (kImg * kImg), r = t - b * kImg * kImg;
         const int q = q64(r / kImg, r % kImg);
-        const float d = out[((size_t)b * kP64 + q) * 16] - target[t];
+        const float d = out[t] - target[t];
         s += (double)d * d;
         const float g = 2.0f * d * scale;
         __nv_bfloat162 h = __floats2bfloat162_rn(g, 0.0f);
@@ -199,14 +199,6 @@ __global__ void k_gather(const uint4* __restrict__ x_all, const float* __restric
         x0[(size_t)k * kP64 * 2 + i] = x_all[src * kP64 * 2 + i];
     for (int i = (int)threadIdx.x; i < kImg * kImg; i += blockDim.x)
         t[(size_t)k * kImg * kImg + i] = t_all[src * kImg * kImg + i];
-}
-
-__global__ void k_take_ch0(const float* __restrict__ out, float* __restrict__ d, int B) {
-    const int n = B * kImg * kImg;
-    for (int t = (int)(blockIdx.x * blockDim.x + threadIdx.x); t < n; t += gridDim.x * blockDim.x) {
-        const int b = t / (kImg * kImg), r = t - b * kImg * kImg;
-        d[t] = out[((size_t)b * kP64 + q64(r / kImg, r % kImg)) * 16];
-    }
 }
 
 int ew_blocks(long long n) {
@@ -254,11 +246,10 @@ struct pfb_sur2d {
     // activations and gradients (padded channels-last), max_batch images
     bf16 *x0 = nullptr, *a1 = nullptr, *a2 = nullptr, *p = nullptr, *a3 = nullptr, *a4 = nullptr,
          *u = nullptr, *a5 = nullptr, *a6 = nullptr, *a7 = nullptr;
-    float* out = nullptr;
+    float* out = nullptr;  // channel 0 of the output, no border
     bf16 *go = nullptr, *dz7 = nullptr, *dz6 = nullptr, *dz5 = nullptr, *gu = nullptr,
          *dz4 = nullptr, *dz3 = nullptr, *gp = nullptr, *dz2 = nullptr, *dz1 = nullptr;
     float* target = nullptr;
-    float* dphi = nullptr;
     int* origins = nullptr;
     double* loss_partial = nullptr;
     float* wg_ws = nullptr;
@@ -307,13 +298,13 @@ struct pfb_sur2d {
             (rc = alloc(&a3, B * kP32 * 32)) || (rc = alloc(&a4, B * kP32 * 32)) ||
             (rc = alloc(&u, B * kP64 * 32)) || (rc = alloc(&a5, B * kP64 * 32)) ||
             (rc = alloc(&a6, B * kP64 * 32)) || (rc = alloc(&a7, B * kP64 * 32)) ||
-            (rc = alloc(&out, B * kP64 * 16)) || (rc = alloc(&go, B * kP64 * 16)) ||
+            (rc = alloc(&out, B * kImg * kImg)) || (rc = alloc(&go, B * kP64 * 16)) ||
             (rc = alloc(&dz7, B * kP64 * 32)) || (rc = alloc(&dz6, B * kP64 * 32)) ||
             (rc = alloc(&dz5, B * kP64 * 32)) || (rc = alloc(&gu, B * kP64 * 32)) ||
             (rc = alloc(&dz4, B * kP32 * 32)) || (rc = alloc(&dz3, B * kP32 * 32)) ||
             (rc = alloc(&gp, B * kP32 * 32)) || (rc = alloc(&dz2, B * kP64 * 32)) ||
             (rc = alloc(&dz1, B * kP64 * 32)) || (rc = alloc(&target, B * kImg * kImg)) ||
-            (rc = alloc(&dphi, B * kImg * kImg)) || (rc = alloc(&origins, B * 2)) ||
+            (rc = alloc(&origins, B * 2)) ||
             (rc = alloc(&loss_partial, (size_t)kLossBlocks)))
             return rc;
         // partial sums of the weight gradients: one block per SM, also for
@@ -340,19 +331,21 @@ struct pfb_sur2d {
         return repack(stream);
     }
 
+    // every layer's packed weights, in one launch
     int repack(cudaStream_t s) {
-        for (int l = 0; l < 8; ++l) {
-            int rc = conv3x3_pack(params + w_off[l], wf[l], kLayers[l].cin, kLayers[l].cout, 0, s);
-            if (!rc && l > 0) rc = conv3x3_pack(params + w_off[l], wd[l], kLayers[l].cin, kLayers[l].cout, 1, s);
-            if (rc) return rc;
-        }
-        return PFB_OK;
+        ConvPackJob jobs[16];
+        int n = 0;
+        for (int l = 0; l < 8; ++l)
+            for (int t = 0; t < (l > 0 ? 2 : 1); ++t)
+                jobs[n++] = ConvPackJob{params + w_off[l], t ? wd[l] : wf[l], kLayers[l].cin, kLayers[l].cout, t};
+        return conv3x3_pack_many(jobs, n, s);
     }
 
-    int conv(int l, const bf16* in, bf16* o, float* of, int B, cudaStream_t s) {
+    // layer l: all channels into o, or channel 0 alone in binary32 into o0
+    int conv(int l, const bf16* in, bf16* o, int B, cudaStream_t s, float* o0 = nullptr) {
         const LayerSpec& L = kLayers[l];
-        return conv3x3_fwd(in, o, of, wf[l], params + b_off[l], nullptr, B, L.res, L.res, L.cin,
-                           L.cout, L.relu, s);
+        return conv3x3_fwd(in, o, nullptr, wf[l], params + b_off[l], nullptr, B, L.res, L.res, L.cin,
+                           L.cout, L.relu, s, o0);
     }
     // data gradient of layer l: dY (cout channels) -> dX (cin), gated by the
     // ReLU of the layer's input when it is one
@@ -366,17 +359,18 @@ struct pfb_sur2d {
                              L.res, L.cin, L.cout, s);
     }
 
-    int forward(const bf16* in, int B, cudaStream_t s) {
+    // The network on B crops; the increments ([B][64][64]) go to res.
+    int forward(const bf16* in, float* res, int B, cudaStream_t s) {
         int rc;
-        if ((rc = conv(0, in, a1, nullptr, B, s)) || (rc = conv(1, a1, a2, nullptr, B, s))) return rc;
+        if ((rc = conv(0, in, a1, B, s)) || (rc = conv(1, a1, a2, B, s))) return rc;
         k_pool2<<<ew_blocks((long long)B * kHalf * kHalf * 4), kEwThreads, 0, s>>>(
             reinterpret_cast<const uint4*>(a2), reinterpret_cast<uint4*>(p), B);
-        if ((rc = conv(2, p, a3, nullptr, B, s)) || (rc = conv(3, a3, a4, nullptr, B, s))) return rc;
+        if ((rc = conv(2, p, a3, B, s)) || (rc = conv(3, a3, a4, B, s))) return rc;
         k_upadd<<<ew_blocks((long long)B * kImg * kImg * 4), kEwThreads, 0, s>>>(
             reinterpret_cast<const uint4*>(a4), reinterpret_cast<const uint4*>(a2),
             reinterpret_cast<uint4*>(u), B);
-        if ((rc = conv(4, u, a5, nullptr, B, s)) || (rc = conv(5, a5, a6, nullptr, B, s)) ||
-            (rc = conv(6, a6, a7, nullptr, B, s)) || (rc = conv(7, a7, nullptr, out, B, s)))
+        if ((rc = conv(4, u, a5, B, s)) || (rc = conv(5, a5, a6, B, s)) ||
+            (rc = conv(6, a6, a7, B, s)) || (rc = conv(7, a7, nullptr, B, s, res)))
             return rc;
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? PFB_OK : set_error(PFB_E_CUDA, "forward: %s", cudaGetErrorString(e));
@@ -469,10 +463,8 @@ int pfb_sur2d_predict(pfb_sur2d* n, const void* x0, float* dphi, int batch) {
     for (int b0 = 0; b0 < batch; b0 += n->max_batch) {
         const int B = batch - b0 < n->max_batch ? batch - b0 : n->max_batch;
         const bf16* in = static_cast<const bf16*>(x0) + (size_t)b0 * kP64 * 16;
-        int rc = n->forward(in, B, n->stream);
+        int rc = n->forward(in, dphi + (size_t)b0 * kImg * kImg, B, n->stream);
         if (rc) return rc;
-        k_take_ch0<<<ew_blocks((long long)B * kImg * kImg), kEwThreads, 0, n->stream>>>(
-            n->out, dphi + (size_t)b0 * kImg * kImg, B);
     }
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PFB_OK : set_error(PFB_E_CUDA, "predict: %s", cudaGetErrorString(e));
@@ -480,7 +472,7 @@ int pfb_sur2d_predict(pfb_sur2d* n, const void* x0, float* dphi, int batch) {
 
 // Loss and gradients of one batch without an update (the gradient check).
 static int loss_and_grads(pfb_sur2d* n, int B, double* loss) {
-    int rc = n->forward(n->x0, B, n->stream);
+    int rc = n->forward(n->x0, n->out, B, n->stream);
     if (rc) return rc;
     k_loss<<<kLossBlocks, kEwThreads, 0, n->stream>>>(n->out, n->target, reinterpret_cast<uint4*>(n->go),
                                                       n->loss_partial, B,
@@ -563,10 +555,7 @@ int pfb_sur2d_jump_history(pfb_sur2d* n, pfb_sim2d* s, int history_steps, float 
     }
     for (int b0 = 0; !rc && b0 < N; b0 += n->max_batch) {
         const int B = N - b0 < n->max_batch ? N - b0 : n->max_batch;
-        rc = n->forward(xin + (size_t)b0 * kP64 * 16, B, v.stream);
-        if (!rc)
-            k_take_ch0<<<ew_blocks((long long)B * kImg * kImg), kEwThreads, 0, v.stream>>>(
-                n->out, d + (size_t)b0 * kImg * kImg, B);
+        rc = n->forward(xin + (size_t)b0 * kP64 * 16, d + (size_t)b0 * kImg * kImg, B, v.stream);
     }
     if (!rc) rc = relax_insert(s, org, d);
     cudaFreeAsync(xin, v.stream);
@@ -588,13 +577,13 @@ int pfb_sur2d_bench_forward(pfb_sur2d* n, int batch, int iters, double* ms) {
     if (!n || batch < 1 || batch > n->max_batch || iters < 1 || !ms)
         return set_error(PFB_E_ARG, "bench_forward: bad argument");
     SUR_CU(cudaSetDevice(n->device), "cudaSetDevice");
-    int rc = n->forward(n->x0, batch, n->stream);
+    int rc = n->forward(n->x0, n->out, batch, n->stream);
     if (rc) return rc;
     cudaEvent_t e0, e1;
     SUR_CU(cudaEventCreate(&e0), "event");
     SUR_CU(cudaEventCreate(&e1), "event");
     cudaEventRecord(e0, n->stream);
-    for (int i = 0; i < iters && !rc; ++i) rc = n->forward(n->x0, batch, n->stream);
+    for (int i = 0; i < iters && !rc; ++i) rc = n->forward(n->x0, n->out, batch, n->stream);
     cudaEventRecord(e1, n->stream);
     const cudaError_t e = cudaEventSynchronize(e1);
     float t = 0.0f;
