@@ -81,10 +81,11 @@ __device__ __forceinline__ void row6v(const T* plane, int B, int ys, int xs0, bo
 }
 
 // stencil27w over a window whose rows rotate through slots: row offset -1,
-// 0, +1 of every plane live in slots s0, s1, s2.
+// 0, +1 of every plane live in slots s0, s1, s2. The sum's rounding is written
+// out (left as + and *, pairs of columns were compiled to other roundings).
 __device__ __forceinline__ float laplace27r(const float (&w)[3][3][6], int s0, int s1, int s2, int j) {
     const int sl[3] = {s0, s1, s2};
-    float acc = (float)kWCentre * w[1][s1][j + 1];
+    float acc = __fmul_rn((float)kWCentre, w[1][s1][j + 1]);
 #pragma unroll
     for (int dz = 0; dz < 3; ++dz)
 #pragma unroll
@@ -94,9 +95,9 @@ __device__ __forceinline__ float laplace27r(const float (&w)[3][3][6], int s0, i
                 const int d = (dz != 1) + (dy != 1) + (dx != 1);
                 if (d == 0) continue;
                 const int wgt = d == 1 ? kWFace : d == 2 ? kWEdge : kWCorner;
-                acc += (float)wgt * w[dz][sl[dy]][j + dx];
+                acc = __fmaf_rn((float)wgt, w[dz][sl[dy]][j + dx], acc);
             }
-    return acc * (float)(1.0 / 30.0);
+    return __fmul_rn(acc, (float)(1.0 / 30.0));
 }
 
 __device__ __forceinline__ void stencil27r(const float (&w)[3][3][6], int s0, int s1, int s2,
