@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kThreads3, 2) k_measure3d(const __grid_constan
     const int strips = B / 4;
     const int items = strips * (B / 4);
 
-    for (int i = 0; i < PB; ++i) {
+    const int eighth = B / kFoldRecords;
+    for (int i = 0, sub = 0, left = eighth; i < PB; ++i) {
         const int z = z0 + i;
         if (!ring.wait(i + 2)) {
             H.abort = 1;
@@ -114,6 +115,10 @@ __global__ void __launch_bounds__(kThreads3, 2) k_measure3d(const __grid_constan
             for (int it = tid; it < items; it += kThreads3)
                 measure_item(M, ring.slot(i), ring.slot(i + 1), ring.slot(i + 2), 4 * (it % strips),
                              4 * (it / strips), z, wz, wallv, top_plane, acc, mc);
+        }
+        if (--left == 0) {
+            fold_sums<K>(H.fold, sub++, acc);
+            left = eighth;
         }
         __syncthreads();
         // after a timed-out wait nothing more is issued into the ring
@@ -221,9 +226,29 @@ static int measure_launch_k(const pfb_measure_args3d& A, int count, cudaStream_t
     return PFB_OK;
 }
 
-// The measurement's cluster size: 4, as the fused step's, so the two paths
-// sum the moments in the same grouping.
-int measure3d_cluster(int) { return 4; }
+// Parts to cut each of `cells` cells into: as many, from `least` to `most`, as
+// still run in one wave at two CTAs per SM. A part stages two halo planes more
+// than it owns, so cells that fill the SMs stay at `least`. 12 channel cells
+// (B = 64), four steps: 718 us at 4 parts, 363 us with this rule (clusters of 8,
+// 16 update parts); 512 cells keep 4.
+int parts_in_one_wave3d(int cells, int least, int most) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return least;
+    const int p = 2 * sms / (cells > 0 ? cells : 1);
+    return p < least ? least : p > most ? most : p;
+}
+
+// The measurement's cluster size. 4 where the cells fill the SMs (fewer halo
+// planes and folds); 8 where a system of few cells would leave SMs idle.
+int measure3d_cluster(int cells) { return parts_in_one_wave3d(cells, 4, 8) == 8 ? 8 : 4; }
+
+template <typename T>
+static int measure_launch_t(const pfb_measure_args3d& A, int count, cudaStream_t stream) {
+    return measure3d_cluster(count) == 8 ? measure_launch_k<8, T>(A, count, stream)
+                                         : measure_launch_k<4, T>(A, count, stream);
+}
 
 int measure3d_launch(const pfb_measure_args3d* a, cudaStream_t stream) {
     return measure3d_launch_pool(a, kStoreF32, stream);
@@ -235,12 +260,10 @@ int measure3d_launch_pool(const pfb_measure_args3d* a, int storage, cudaStream_t
     const pfb_measure_args3d& A = *a;
     const int count = A.selection.ids ? A.selection.count : A.N;
     if (count == 0) return PFB_OK;
-    const int K = measure3d_cluster(A.B);
-    if (K != 4 || A.B % K != 0) return set_error(PFB_E_CONFIG, "brick edge is not a multiple of 4");
-    if (storage == kStoreF16) return measure_launch_k<4, __half>(A, count, stream);
-    if (storage == kStoreBF16) return measure_launch_k<4, __nv_bfloat16>(A, count, stream);
+    if (storage == kStoreF16) return measure_launch_t<__half>(A, count, stream);
+    if (storage == kStoreBF16) return measure_launch_t<__nv_bfloat16>(A, count, stream);
     if (storage != kStoreF32) return set_error(PFB_E_ARG, "unknown phi storage");
-    return measure_launch_k<4, float>(A, count, stream);
+    return measure_launch_t<float>(A, count, stream);
 }
 
 int motion3d_launch(const pfb_measure_args3d* a, cudaStream_t stream) {

@@ -167,17 +167,23 @@ __device__ __forceinline__ void measure_item(const MeasureCell& M, const T* pm,
 }
 
 // ---- cluster fold -----------------------------------------------------------
-// Bytes one rank pushes into rank 0: 8 sums, 8 integers, 4 counts.
-constexpr uint32_t kFoldBytes = 8 * 8 + 8 * 4 + 4 * 4;
+// The sums are grouped by eighths of the brick's planes whatever the cluster
+// size, so every split of a cell gives the same bits: a rank closes one record
+// of 8 sums per eighth it owns (8 / K of them).
+constexpr int kFoldRecords = 8;
+// Bytes pushed into rank 0: 8 sums per record, 8 integers and 4 counts per rank.
+template <int K>
+constexpr uint32_t kFoldBytes = kFoldRecords * 8 * 8 + K * (8 * 4 + 4 * 4);
 
 template <int K>
 struct MeasureFold {
-    uint64_t bar;  // rank 0: completes when all K records have landed
+    static_assert(kFoldRecords % K == 0, "whole records per rank");
+    uint64_t bar;  // rank 0: completes when every record has landed
     int pad[2];
-    double wd[kWarps3][8];
+    double wd[kFoldRecords / K][kWarps3][8];
     int wi[kWarps3][8];
     unsigned wc[kWarps3][4];
-    alignas(16) double rd[K][8];
+    alignas(16) double rd[kFoldRecords][8];
     alignas(16) int ri[K][8];  // support box (6), phi_max bits, 0
     alignas(16) unsigned rc[K][4];
 };
@@ -194,33 +200,36 @@ struct MeasureTotals {
 template <int K>
 __device__ __forceinline__ void fold_init(MeasureFold<K>& F, int rank) {
     dev::mbar_init(&F.bar, 1);
-    if (rank == 0) dev::mbar_arrive_expect_tx(&F.bar, (uint32_t)K * kFoldBytes);
+    if (rank == 0) dev::mbar_arrive_expect_tx(&F.bar, kFoldBytes<K>);
 }
 
-// Every thread: warp sums of its partial record into F.w*. The caller
-// synchronises the CTA afterwards.
+// Every thread, after the last plane of the rank's eighth `sub`: warp sums of
+// that record, which starts again at zero.
 template <int K>
-__device__ __forceinline__ void fold_warps(MeasureFold<K>& F, Acc3& acc, MeasureCounts c) {
+__device__ __forceinline__ void fold_sums(MeasureFold<K>& F, int sub, Acc3& acc) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* s[8] = {&acc.V, &acc.Cx, &acc.Cy, &acc.Cz, &acc.Sf, &acc.Ix, &acc.Iy, &acc.Iz};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const double v = dev::warp_sum_down(*s[k]);
+        if (lane == 0) F.wd[sub][warp][k] = v;
+        *s[k] = 0.0;
+    }
+}
+
+// Every thread: warp results of the rank's box, maximum and counts. The
+// caller synchronises the CTA afterwards.
+template <int K>
+__device__ __forceinline__ void fold_warps(MeasureFold<K>& F, const Acc3& acc, MeasureCounts c) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     c.nonfinite = __reduce_add_sync(0xFFFFFFFFu, c.nonfinite);
     c.negative = __reduce_add_sync(0xFFFFFFFFu, c.negative);
     c.top = __reduce_add_sync(0xFFFFFFFFu, c.top);
-    acc.V = dev::warp_sum_down(acc.V);
-    acc.Cx = dev::warp_sum_down(acc.Cx);
-    acc.Cy = dev::warp_sum_down(acc.Cy);
-    acc.Cz = dev::warp_sum_down(acc.Cz);
-    acc.Sf = dev::warp_sum_down(acc.Sf);
-    acc.Ix = dev::warp_sum_down(acc.Ix);
-    acc.Iy = dev::warp_sum_down(acc.Iy);
-    acc.Iz = dev::warp_sum_down(acc.Iz);
     const int b0 = __reduce_min_sync(0xFFFFFFFFu, acc.lox), b1 = __reduce_max_sync(0xFFFFFFFFu, acc.hix);
     const int b2 = __reduce_min_sync(0xFFFFFFFFu, acc.loy), b3 = __reduce_max_sync(0xFFFFFFFFu, acc.hiy);
     const int b4 = __reduce_min_sync(0xFFFFFFFFu, acc.loz), b5 = __reduce_max_sync(0xFFFFFFFFu, acc.hiz);
     const unsigned pm = __reduce_max_sync(0xFFFFFFFFu, acc.pmax);
     if (lane == 0) {
-        double* d = F.wd[warp];
-        d[0] = acc.V; d[1] = acc.Cx; d[2] = acc.Cy; d[3] = acc.Cz;
-        d[4] = acc.Sf; d[5] = acc.Ix; d[6] = acc.Iy; d[7] = acc.Iz;
         int* q = F.wi[warp];
         q[0] = b0; q[1] = b1; q[2] = b2; q[3] = b3; q[4] = b4; q[5] = b5; q[6] = (int)pm; q[7] = 0;
         F.wc[warp][0] = c.nonfinite;
@@ -231,15 +240,18 @@ __device__ __forceinline__ void fold_warps(MeasureFold<K>& F, Acc3& acc, Measure
 }
 
 // Warp 0 of every rank, after the CTA barrier and after rank 0's barrier is
-// known to be initialised: the CTA's record (warps in ascending order) is
-// pushed into rank 0's slot `rank`.
+// known to be initialised: the CTA's records (warps in ascending order) are
+// pushed into rank 0's slots.
 template <int K>
 __device__ __forceinline__ void fold_send(MeasureFold<K>& F, int rank, int B) {
     const int lane = threadIdx.x & 31;
-    double s[8];
+    constexpr int RPR = kFoldRecords / K;
+    double s[RPR][8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
-        s[k] = dev::ordered_lane_sum(lane < kWarps3 ? F.wd[lane][k] : 0.0, kWarps3);
+    for (int u = 0; u < RPR; ++u)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            s[u][k] = dev::ordered_lane_sum(lane < kWarps3 ? F.wd[u][lane][k] : 0.0, kWarps3);
     int v[8];
     v[0] = __reduce_min_sync(0xFFFFFFFFu, lane < kWarps3 ? F.wi[lane][0] : B);
     v[1] = __reduce_max_sync(0xFFFFFFFFu, lane < kWarps3 ? F.wi[lane][1] : -1);
@@ -256,9 +268,11 @@ __device__ __forceinline__ void fold_send(MeasureFold<K>& F, int rank, int B) {
     if (lane == 0) {
         const uint32_t bar = dev::map_to_rank(dev::smem_addr(&F.bar), 0);
 #pragma unroll
-        for (int k = 0; k < 8; k += 2)
-            dev::st_async_v2f64(dev::map_to_rank(dev::smem_addr(&F.rd[rank][k]), 0), s[k],
-                                s[k + 1], bar);
+        for (int u = 0; u < RPR; ++u)
+#pragma unroll
+            for (int k = 0; k < 8; k += 2)
+                dev::st_async_v2f64(dev::map_to_rank(dev::smem_addr(&F.rd[rank * RPR + u][k]), 0),
+                                    s[u][k], s[u][k + 1], bar);
         dev::st_async_v4b32(dev::map_to_rank(dev::smem_addr(&F.ri[rank][0]), 0), v[0], v[1],
                             v[2], v[3], bar);
         dev::st_async_v4b32(dev::map_to_rank(dev::smem_addr(&F.ri[rank][4]), 0), v[4], v[5],
@@ -268,7 +282,7 @@ __device__ __forceinline__ void fold_send(MeasureFold<K>& F, int rank, int B) {
     }
 }
 
-// Warp 0 of rank 0: wait for the K records and fold them in rank order.
+// Warp 0 of rank 0: wait for the records and fold them in plane order.
 // false when the wait gave up (the totals are then meaningless).
 template <int K>
 __device__ __forceinline__ bool fold_receive(MeasureFold<K>& F, int B, uint32_t polls,
@@ -276,7 +290,7 @@ __device__ __forceinline__ bool fold_receive(MeasureFold<K>& F, int B, uint32_t 
     const int lane = threadIdx.x & 31;
     const bool ok = dev::mbar_wait_bounded(&F.bar, 0, polls);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) r.t[k] = dev::ordered_lane_sum(lane < K ? F.rd[lane][k] : 0.0, K);
+    for (int k = 0; k < 8; ++k) r.t[k] = dev::ordered_lane_sum(lane < kFoldRecords ? F.rd[lane][k] : 0.0, kFoldRecords);
     r.lo_x = __reduce_min_sync(0xFFFFFFFFu, lane < K ? F.ri[lane][0] : B);
     r.hi_x = __reduce_max_sync(0xFFFFFFFFu, lane < K ? F.ri[lane][1] : -1);
     r.lo_y = __reduce_min_sync(0xFFFFFFFFu, lane < K ? F.ri[lane][2] : B);

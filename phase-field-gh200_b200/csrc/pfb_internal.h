@@ -207,7 +207,7 @@ int check_measure(const pfb_measure_args3d* a);
 // pools = false: the base phi pools are not needed (promoted-cube launches)
 int check_update(const pfb_update_args3d* a, bool pools = true);
 // cluster size of the measurement (the fused step's where it applies)
-int measure3d_cluster(int B);
+int measure3d_cluster(int cells);
 // step3d.cu: fused measure + motion + update; cluster size 0 when the brick
 // does not fit the fused kernel's shared memory
 int step3d_cluster(int B);

@@ -83,18 +83,24 @@ __global__ void __launch_bounds__(kThreads3, 2)
     Acc3 acc;
     acc.lox = acc.loy = acc.loz = E;
     MeasureCounts mc;
-    for (int i = 0; i < PB; ++i) {
+    const int eighth = E / kFoldRecords;
+    for (int i = 0, sub = 0, left = eighth; i < PB; ++i) {
         const int z = z0 + i;
         int wz = 0;
-        if (!aggregate_z(L, oz, z, &wz)) continue;
-        const float* pm = cube_plane(cube, L, oz, z - 1, E);
-        const float* pc = cube_plane(cube, L, oz, z, E);
-        const float* pp = cube_plane(cube, L, oz, z + 1, E);
-        const float wallv = M.wall ? A.wall.values[wz] : 0.0f;
-        const bool top_plane = substrate_slab(bf) && wz == L.nz - 1;
-        for (int it = tid; it < items; it += kThreads3)
-            measure_item(M, pm, pc, pp, 4 * (it % strips), 4 * (it / strips), z, wz, wallv, top_plane,
-                         acc, mc);
+        if (aggregate_z(L, oz, z, &wz)) {
+            const float* pm = cube_plane(cube, L, oz, z - 1, E);
+            const float* pc = cube_plane(cube, L, oz, z, E);
+            const float* pp = cube_plane(cube, L, oz, z + 1, E);
+            const float wallv = M.wall ? A.wall.values[wz] : 0.0f;
+            const bool top_plane = substrate_slab(bf) && wz == L.nz - 1;
+            for (int it = tid; it < items; it += kThreads3)
+                measure_item(M, pm, pc, pp, 4 * (it % strips), 4 * (it / strips), z, wz, wallv, top_plane,
+                             acc, mc);
+        }
+        if (--left == 0) {
+            fold_sums<K>(F, sub++, acc);
+            left = eighth;
+        }
     }
     fold_warps<K>(F, acc, mc);
     __syncthreads();

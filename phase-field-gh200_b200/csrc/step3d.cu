@@ -129,7 +129,8 @@ __global__ void __launch_bounds__(kThreads3, 2) k_step3d(const __grid_constant__
     Acc3 acc;
     acc.lox = acc.loy = acc.loz = B;
     MeasureCounts mc;
-    for (int i = 0; i < PB; ++i) {
+    const int eighth = B / kFoldRecords;
+    for (int i = 0, sub = 0, left = eighth; i < PB; ++i) {
         if (!ring.wait(i + 2)) fail(1u);
         const int z = z0 + i;
         int wz = 0;
@@ -139,6 +140,10 @@ __global__ void __launch_bounds__(kThreads3, 2) k_step3d(const __grid_constant__
             for (int it = tid; it < items; it += kThreads3)
                 measure_item(M, ring.slot(i), ring.slot(i + 1), ring.slot(i + 2), 4 * (it % strips),
                              4 * (it / strips), z, wz, wallv, top_plane, acc, mc);
+        }
+        if (--left == 0) {
+            fold_sums<K>(H.fold, sub++, acc);
+            left = eighth;
         }
         __syncthreads();
         if (!H.fail && issued < nreq) {

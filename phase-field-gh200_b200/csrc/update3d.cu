@@ -31,7 +31,7 @@ namespace p3 {
 
 constexpr int kUThreads = 256;
 constexpr int kURing = 5;
-constexpr int kUCtasPerCell = 4;
+constexpr int kUCtasPerCell = 4;  // where the cells fill the SMs
 
 __device__ unsigned int g_update3d_status = 0u;
 
@@ -54,13 +54,13 @@ struct PoolRounding {
 
 template <int GEO, typename T>
 __global__ void __launch_bounds__(kUThreads, 2)
-    k_update3d(const __grid_constant__ pfb_update_args3d A, int out_by_slot, PoolRounding R) {
+    k_update3d(const __grid_constant__ pfb_update_args3d A, int out_by_slot, int parts, PoolRounding R) {
     extern __shared__ __align__(128) char smem[];
     UpdateHeader& H = *reinterpret_cast<UpdateHeader*>(smem);
     const int B = A.B;
     const int tid = threadIdx.x;
-    const int slot_cell = (int)(blockIdx.x / kUCtasPerCell);
-    const int part = (int)(blockIdx.x % kUCtasPerCell);
+    const int slot_cell = (int)blockIdx.x / parts;
+    const int part = (int)blockIdx.x - slot_cell * parts;
     const int n = A.selection.ids ? A.selection.ids[slot_cell] : slot_cell;
     pfb_cell3d* cell = &A.cells[n];
     if (cell->storage_edge > (uint32_t)B) return;
@@ -68,8 +68,8 @@ __global__ void __launch_bounds__(kUThreads, 2)
     const size_t words = (size_t)B * B * B;
     const T* src = reinterpret_cast<const T*>(A.phi_in) + (size_t)n * words;
     T* dst = reinterpret_cast<T*>(A.phi_out) + (size_t)(out_by_slot ? slot_cell : n) * words;
-    const int PB = B / kUCtasPerCell;
-    const int d0 = part * PB, d1 = d0 + PB;
+    const int d0 = part * B / parts, d1 = (part + 1) * B / parts;
+    const int PB = d1 - d0;
     const int64_t oz = cell->origin_z;
     const uint32_t sr = Store<T>::kHalf ? sr_stream(R.step ? *R.step : 0ull, cell->global_id, R.seed) : 0u;
 
@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(kUThreads, 2)
 // Host side
 // ---------------------------------------------------------------------------
 int geometry_ok3(int B, const pfb_layout3d& L);
+int parts_in_one_wave3d(int cells, int least, int most);
 
 size_t update3d_smem(int B, int bytes = 4) {
     return (size_t)kUHeader + (size_t)kURing * (size_t)B * B * bytes;
@@ -203,21 +204,21 @@ int check_update(const pfb_update_args3d* a, bool pools) {
 }
 
 template <int GEO, typename T>
-static cudaError_t update_launch_gt(const pfb_update_args3d& A, int out_by_slot, PoolRounding R,
+static cudaError_t update_launch_gt(const pfb_update_args3d& A, int out_by_slot, PoolRounding R, int parts,
                                     dim3 grid, size_t smem, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(k_update3d<GEO, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
-    if (e == cudaSuccess) k_update3d<GEO, T><<<grid, kUThreads, smem, stream>>>(A, out_by_slot, R);
+    if (e == cudaSuccess) k_update3d<GEO, T><<<grid, kUThreads, smem, stream>>>(A, out_by_slot, parts, R);
     return e;
 }
 
 template <typename T>
-static cudaError_t update_launch_t(const pfb_update_args3d& A, int out_by_slot, PoolRounding R, dim3 grid,
-                                   size_t smem, cudaStream_t stream) {
+static cudaError_t update_launch_t(const pfb_update_args3d& A, int out_by_slot, PoolRounding R, int parts,
+                                   dim3 grid, size_t smem, cudaStream_t stream) {
     const uint32_t bf = A.layout.boundary_flags;
-    if (periodic_xyz(bf)) return update_launch_gt<0, T>(A, out_by_slot, R, grid, smem, stream);
-    if (substrate_slab(bf)) return update_launch_gt<1, T>(A, out_by_slot, R, grid, smem, stream);
-    return update_launch_gt<2, T>(A, out_by_slot, R, grid, smem, stream);
+    if (periodic_xyz(bf)) return update_launch_gt<0, T>(A, out_by_slot, R, parts, grid, smem, stream);
+    if (substrate_slab(bf)) return update_launch_gt<1, T>(A, out_by_slot, R, parts, grid, smem, stream);
+    return update_launch_gt<2, T>(A, out_by_slot, R, parts, grid, smem, stream);
 }
 
 static int update_launch(const pfb_update_args3d& A, int out_by_slot, int storage, PoolRounding R,
@@ -226,14 +227,18 @@ static int update_launch(const pfb_update_args3d& A, int out_by_slot, int storag
     if (count == 0) return PFB_OK;
     const size_t smem = update3d_smem(A.B, storage ? 2 : 4);
     if (smem > 227 * 1024) return set_error(PFB_E_CONFIG, "brick edge too large for the plane ring");
-    const dim3 grid((unsigned)(count * kUCtasPerCell));
+    // a few cells are cut into more parts (of 4 planes at least: each part
+    // stages two planes more than it updates) so that the SMs are not idle;
+    // the result does not depend on the cut
+    const int parts = parts_in_one_wave3d(count, kUCtasPerCell, A.B / 4 > kUCtasPerCell ? A.B / 4 : kUCtasPerCell);
+    const dim3 grid((unsigned)(count * parts));
     cudaError_t e;
     if (storage == kStoreF16)
-        e = update_launch_t<__half>(A, out_by_slot, R, grid, smem, stream);
+        e = update_launch_t<__half>(A, out_by_slot, R, parts, grid, smem, stream);
     else if (storage == kStoreBF16)
-        e = update_launch_t<__nv_bfloat16>(A, out_by_slot, R, grid, smem, stream);
+        e = update_launch_t<__nv_bfloat16>(A, out_by_slot, R, parts, grid, smem, stream);
     else
-        e = update_launch_t<float>(A, out_by_slot, R, grid, smem, stream);
+        e = update_launch_t<float>(A, out_by_slot, R, parts, grid, smem, stream);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(PFB_E_CUDA, "update launch: %s", cudaGetErrorString(e));
     return PFB_OK;
