@@ -22,8 +22,6 @@ constexpr int kDefaultCluster = 2;
 int step2d_smem_bytes(int cluster);
 // Systems r = 0..R-1 in one launch: d_args[r] (device) is served by CTAs
 // [d_block_start[r], d_block_start[r+1]) (R+1 entries, multiples of cluster).
-int step2d_launch_batch(const pfb_step_args2d* d_args, const int* d_block_start, int R,
-                        int total_blocks, int cluster, int storage, cudaStream_t stream);
 int step2d_read_status(unsigned* out, int clear);
 int init2d_read_status(unsigned* out, int clear);
 // variant: 0 = default, 1 = one thread-block cluster per cell
@@ -53,6 +51,13 @@ int step2d_launch_binned(const pfb_step_args2d* a, int cluster, int storage, con
 // storage 0/1/2) and raises S_overflow when some pixel total reaches 2^32.
 int step2d_settle_bins(const BinArgs& B, const void* phi, int storage, int N, int L,
                        unsigned long long step, uint32_t* flags, cudaStream_t stream);
+// R systems in one launch, and the settling of their last launch's bounds
+// (d_next: the arguments of their next step). Tables in device memory.
+int step2d_launch_batch(const pfb_step_args2d* d_args, const BinArgs* d_bins,
+                        const int* d_block_start, int R, int total_blocks, int cluster, int storage,
+                        cudaStream_t stream);
+int step2d_settle_batch(const pfb_step_args2d* d_next, const BinArgs* d_bins, int R, int storage,
+                        cudaStream_t stream);
 // The step with a velocity observer (PFB_VELOCITY_*), binary32 pools.
 int step2d_launch_observed(const pfb_step_args2d* a, int cluster, int observation,
                            cudaStream_t stream);

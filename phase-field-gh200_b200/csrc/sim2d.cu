@@ -1010,6 +1010,7 @@ struct pfb_ens2d {
     long long steps_done = 0;
     cudaStream_t stream = nullptr;
     pfb_step_args2d* d_args = nullptr;  // 6 slots x R records
+    BinArgs* d_bins = nullptr;          // R records, launch order
     int* d_start = nullptr;             // R + 1 block offsets
     int total_blocks = 0;
     bool tables_ready = false;
@@ -1028,6 +1029,7 @@ struct pfb_ens2d {
         drop_graph();
         if (stream) cudaStreamDestroy(stream);
         cudaFree(d_args);
+        cudaFree(d_bins);
         cudaFree(d_start);
         cudaFree(d_src);
         cudaFree(d_ring);
@@ -1146,7 +1148,7 @@ struct pfb_ens2d {
             }
         }
         for (pfb_sim2d* s : sims) s->steps_done = steps_done;
-        return PFB_OK;
+        return steps > 0 ? settle() : PFB_OK;
     }
 
     // Argument tables for the six slots and the CTA offsets for `cluster`.
@@ -1154,15 +1156,20 @@ struct pfb_ens2d {
         drop_graph();
         const int R_ = R();
         std::vector<pfb_step_args2d> h((size_t)6 * R_);
+        std::vector<BinArgs> bins((size_t)R_);
         std::vector<int> start((size_t)R_ + 1, 0);
         for (int i = 0; i < R_; ++i) {
             const pfb_sim2d* s = sims[(size_t)order[(size_t)i]];
+            bins[(size_t)i] = s->bin_args();
             for (int slot = 0; slot < 6; ++slot) h[(size_t)slot * R_ + i] = s->args_for_slot(slot);
             start[(size_t)i + 1] = start[(size_t)i] + s->N * cluster;
         }
         total_blocks = start[(size_t)R_];
         if (!d_args) PFB_CU(cudaMalloc(&d_args, h.size() * sizeof(pfb_step_args2d)), "alloc args");
+        if (!d_bins) PFB_CU(cudaMalloc(&d_bins, bins.size() * sizeof(BinArgs)), "alloc bin table");
         if (!d_start) PFB_CU(cudaMalloc(&d_start, start.size() * sizeof(int)), "alloc offsets");
+        PFB_CU(cudaMemcpyAsync(d_bins, bins.data(), bins.size() * sizeof(BinArgs),
+                               cudaMemcpyHostToDevice, stream), "upload bin table");
         PFB_CU(cudaMemcpyAsync(d_args, h.data(), h.size() * sizeof(pfb_step_args2d),
                                cudaMemcpyHostToDevice, stream), "upload args");
         PFB_CU(cudaMemcpyAsync(d_start, start.data(), start.size() * sizeof(int),
@@ -1173,8 +1180,14 @@ struct pfb_ens2d {
     }
 
     int launch_slot(int slot) {
-        return step2d_launch_batch(d_args + (size_t)slot * R(), d_start, R(), total_blocks, cluster,
-                                   storage, stream);
+        return step2d_launch_batch(d_args + (size_t)slot * R(), d_bins, d_start, R(), total_blocks,
+                                   cluster, storage, stream);
+    }
+
+    // Settle the bounds of the last batch launch: the flags are final when an
+    // advance ends, and every other path finds both sets clear.
+    int settle() {
+        return step2d_settle_batch(d_args + (size_t)(steps_done % 6) * R(), d_bins, R(), storage, stream);
     }
 
     int build_graph() {
@@ -1199,6 +1212,7 @@ struct pfb_ens2d {
             const int rc = build_tables();
             if (rc) return rc;
         }
+        const bool ran = steps > 0;
         while (steps > 0) {
             if (steps_done % 6 == 0 && steps >= 6) {
                 if (!graph_exec) {
@@ -1216,7 +1230,7 @@ struct pfb_ens2d {
             }
         }
         for (pfb_sim2d* s : sims) s->steps_done = steps_done;
-        return PFB_OK;
+        return ran ? settle() : PFB_OK;
     }
 
     // The same steps with one launch per system (the replicas-one-at-a-time

@@ -882,13 +882,15 @@ __global__ void __launch_bounds__(kThreads, min_blocks(K))
 // Many independent systems in one launch: system r is served by CTAs
 // [block_start[r], block_start[r+1]) (multiples of K, so clusters never
 // straddle systems); its arguments are copied into shared memory. All
-// systems of one launch share the pool storage type T.
+// systems of one launch share the pool storage type T. The scatter is the
+// non-returning one under each system's own bin bounds.
 template <int K, typename T = float>
 __global__ void __launch_bounds__(kThreads, min_blocks(K))
-    k_step2d_batch(const pfb_step_args2d* __restrict__ args, const int* __restrict__ block_start,
-                   int R) {
+    k_step2d_batch(const pfb_step_args2d* __restrict__ args, const BinArgs* __restrict__ bins,
+                   const int* __restrict__ block_start, int R) {
     extern __shared__ __align__(128) char smem[];
     __shared__ __align__(16) pfb_step_args2d sA;
+    __shared__ __align__(16) BinArgs sB;
     const int b = (int)blockIdx.x;
     int lo = 0, hi = R - 1;  // last r with block_start[r] <= b
     while (lo < hi) {
@@ -903,9 +905,13 @@ __global__ void __launch_bounds__(kThreads, min_blocks(K))
     const uint64_t* srcw = reinterpret_cast<const uint64_t*>(args + r);
     uint64_t* dstw = reinterpret_cast<uint64_t*>(&sA);
     if (threadIdx.x < sizeof(pfb_step_args2d) / 8) dstw[threadIdx.x] = __ldg(srcw + threadIdx.x);
+    static_assert(sizeof(BinArgs) % 8 == 0, "bin record copy");
+    if (threadIdx.x < sizeof(BinArgs) / 8)
+        reinterpret_cast<uint64_t*>(&sB)[threadIdx.x] =
+            __ldg(reinterpret_cast<const uint64_t*>(bins + r) + threadIdx.x);
     __syncthreads();
     const int b0 = __ldg(block_start + r);
-    step_body<K, T>(sA, b - b0, __ldg(block_start + r + 1) - b0, smem);
+    step_body<K, T, PFB_VELOCITY_DISABLED, true>(sA, b - b0, __ldg(block_start + r + 1) - b0, smem, sB);
 }
 
 // ---------------------------------------------------------------------------
@@ -1107,6 +1113,40 @@ int step2d_settle_bins(const BinArgs& B, const void* phi, int storage, int N, in
     return PFB_OK;
 }
 
+// Row r of the grid settles system r: args[r] are the arguments of its next
+// step (phi_in is the field the last launch wrote).
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    k_settle_bins2d_batch(const pfb_step_args2d* __restrict__ args, const BinArgs* __restrict__ bins) {
+    __shared__ __align__(16) char scratch[256 * sizeof(unsigned long long) + (kThreads + 1) * 4];
+    const pfb_step_args2d& A = args[blockIdx.y];
+    const BinArgs B = bins[blockIdx.y];
+    const int nbins = B.nbx * B.nby;
+    const int par = (int)((*A.step_rd - 1ull) & 1ull);
+    for (int first = blockIdx.x * kThreads; first < nbins; first += gridDim.x * kThreads)
+        bin_settle_chunk<T>(B.bound + (size_t)par * nbins, B.geo + (size_t)par * A.N,
+                            reinterpret_cast<const T*>(A.phi_in), A.N, A.L, B.nbx, first,
+                            min(kThreads, nbins - first), A.flags, B.recounts, scratch);
+}
+
+int step2d_settle_batch(const pfb_step_args2d* d_next, const BinArgs* d_bins, int R, int storage,
+                        cudaStream_t stream) {
+    if (!d_next || !d_bins || R <= 0) return set_error(PFB_E_ARG, "settle_bins: bad arguments");
+    // a system has at most a few thousand bins
+    for (int r0 = 0; r0 < R; r0 += 65535) {
+        const dim3 grid(4u, (unsigned)std::min(R - r0, 65535));
+        if (storage == kStoreF16)
+            k_settle_bins2d_batch<__half><<<grid, kThreads, 0, stream>>>(d_next + r0, d_bins + r0);
+        else if (storage == kStoreBF16)
+            k_settle_bins2d_batch<__nv_bfloat16><<<grid, kThreads, 0, stream>>>(d_next + r0, d_bins + r0);
+        else
+            k_settle_bins2d_batch<float><<<grid, kThreads, 0, stream>>>(d_next + r0, d_bins + r0);
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return set_error(PFB_E_CUDA, "settle_bins: %s", cudaGetErrorString(e));
+    return PFB_OK;
+}
+
 int step2d_launch_observed(const pfb_step_args2d* a, int cluster, int observation,
                            cudaStream_t stream) {
     if (observation == PFB_VELOCITY_DISABLED) {
@@ -1147,8 +1187,9 @@ int step2d_launch_variant(const pfb_step_args2d* a, int cluster, int variant,
 }
 
 template <int K, typename T = float>
-static cudaError_t launch_batch_k(const pfb_step_args2d* args, const int* block_start, int R,
-                                  int total_blocks, cudaStream_t stream) {
+static cudaError_t launch_batch_k(const pfb_step_args2d* args, const BinArgs* bins,
+                                  const int* block_start, int R, int total_blocks,
+                                  cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)total_blocks, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -1161,12 +1202,13 @@ static cudaError_t launch_batch_k(const pfb_step_args2d* args, const int* block_
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_step2d_batch<K, T>, args, block_start, R);
+    return cudaLaunchKernelEx(&cfg, k_step2d_batch<K, T>, args, bins, block_start, R);
 }
 
-int step2d_launch_batch(const pfb_step_args2d* d_args, const int* d_block_start, int R,
-                        int total_blocks, int cluster, int storage, cudaStream_t stream) {
-    if (!d_args || !d_block_start || R <= 0 || total_blocks < 0)
+int step2d_launch_batch(const pfb_step_args2d* d_args, const BinArgs* d_bins,
+                        const int* d_block_start, int R, int total_blocks, int cluster, int storage,
+                        cudaStream_t stream) {
+    if (!d_args || !d_bins || !d_block_start || R <= 0 || total_blocks < 0)
         return set_error(PFB_E_ARG, "invalid batch arguments");
     if (cluster == 0) cluster = kDefaultCluster;
     if (cluster != 2 && cluster != 4 && cluster != 8)
@@ -1180,16 +1222,16 @@ int step2d_launch_batch(const pfb_step_args2d* d_args, const int* d_block_start,
     if (rc) return rc;
     cudaError_t e;
     if (storage == kStoreF16)
-        e = cluster == 2 ? launch_batch_k<2, __half>(d_args, d_block_start, R, total_blocks, stream)
-                         : launch_batch_k<4, __half>(d_args, d_block_start, R, total_blocks, stream);
+        e = cluster == 2 ? launch_batch_k<2, __half>(d_args, d_bins, d_block_start, R, total_blocks, stream)
+                         : launch_batch_k<4, __half>(d_args, d_bins, d_block_start, R, total_blocks, stream);
     else if (storage == kStoreBF16)
         e = cluster == 2
-                ? launch_batch_k<2, __nv_bfloat16>(d_args, d_block_start, R, total_blocks, stream)
-                : launch_batch_k<4, __nv_bfloat16>(d_args, d_block_start, R, total_blocks, stream);
+                ? launch_batch_k<2, __nv_bfloat16>(d_args, d_bins, d_block_start, R, total_blocks, stream)
+                : launch_batch_k<4, __nv_bfloat16>(d_args, d_bins, d_block_start, R, total_blocks, stream);
     else
-        e = cluster == 2   ? launch_batch_k<2>(d_args, d_block_start, R, total_blocks, stream)
-            : cluster == 4 ? launch_batch_k<4>(d_args, d_block_start, R, total_blocks, stream)
-                           : launch_batch_k<8>(d_args, d_block_start, R, total_blocks, stream);
+        e = cluster == 2   ? launch_batch_k<2>(d_args, d_bins, d_block_start, R, total_blocks, stream)
+            : cluster == 4 ? launch_batch_k<4>(d_args, d_bins, d_block_start, R, total_blocks, stream)
+                           : launch_batch_k<8>(d_args, d_bins, d_block_start, R, total_blocks, stream);
     if (e != cudaSuccess) return set_error(PFB_E_CUDA, "batch launch: %s", cudaGetErrorString(e));
     return PFB_OK;
 }
