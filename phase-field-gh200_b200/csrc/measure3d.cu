@@ -229,8 +229,8 @@ static int measure_launch_k(const pfb_measure_args3d& A, int count, cudaStream_t
 // Parts to cut each of `cells` cells into: as many, from `least` to `most`, as
 // still run in one wave at two CTAs per SM. A part stages two halo planes more
 // than it owns, so cells that fill the SMs stay at `least`. 12 channel cells
-// (B = 64), four steps: 718 us at 4 parts, 363 us with this rule (clusters of 8,
-// 16 update parts); 512 cells keep 4.
+// (B = 64), four steps: 718 us at 4 parts, 333 us with this rule (clusters of 8,
+// 24 update parts; 363 us at 16); 512 cells keep 4.
 int parts_in_one_wave3d(int cells, int least, int most) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||

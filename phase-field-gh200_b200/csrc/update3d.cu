@@ -227,10 +227,10 @@ static int update_launch(const pfb_update_args3d& A, int out_by_slot, int storag
     if (count == 0) return PFB_OK;
     const size_t smem = update3d_smem(A.B, storage ? 2 : 4);
     if (smem > 227 * 1024) return set_error(PFB_E_CONFIG, "brick edge too large for the plane ring");
-    // a few cells are cut into more parts (of 4 planes at least: each part
+    // a few cells are cut into more parts (of 2 planes at least: each part
     // stages two planes more than it updates) so that the SMs are not idle;
     // the result does not depend on the cut
-    const int parts = parts_in_one_wave3d(count, kUCtasPerCell, A.B / 4 > kUCtasPerCell ? A.B / 4 : kUCtasPerCell);
+    const int parts = parts_in_one_wave3d(count, kUCtasPerCell, A.B / 2);
     const dim3 grid((unsigned)(count * parts));
     cudaError_t e;
     if (storage == kStoreF16)
