@@ -474,9 +474,16 @@ __global__ void __launch_bounds__(kWsThreads)
 // or nine of one tap each would be bound by their number.
 //
 // Warp-specialised and persistent, one CTA per SM: CTA c owns a contiguous
-// range of the B x chunks tiles and accumulates all of it in TMEM; warp 0
-// keeps a ring of kWgStages tiles in flight, warp 1 issues, warps 2-5 write
-// the CTA's partial sums at the end. 256 crops of 64 x 64, 32 -> 32
+// range of the B x chunks tiles; warp 0 keeps a ring of kWgStages tiles in
+// flight, warp 1 issues, and warps 2-5 take the accumulator out of TMEM after
+// every run of `run` tiles, add it to the CTA's sums in registers and write
+// those at the end. The tensor core adds into its accumulator with a bias
+// towards zero, so the error of one-signed sums grows with the length of the
+// chain: 2.7e-5 of the gradient over a CTA's whole range at 256 crops of
+// 64 x 64 (457 additions), 5.6e-6 over half an image (132), 1.0e-6 over the 36
+// of a run. Two accumulators keep the MMAs going meanwhile (a layer of 256
+// crops takes 51.8 us with the reduction, 49.3 us in one chain, launches back
+// to back). 256 crops of 64 x 64, 32 -> 32
 // channels: 52 us a layer with the reduction, against about 200 of one CTA per
 // half image that staged nine shifted copies of x with cp.async; bound by the
 // TMA fill (392 rows per tile, 1.3 GB a layer through the L2).
@@ -484,7 +491,8 @@ constexpr int kWgStages = 6;
 constexpr int kWgThreads = 192;
 constexpr int kWgKT = 96;        // positions per tile: divides 64 x 66 exactly
 constexpr int kWgHeader = 1024;  // barriers
-constexpr uint32_t kWgCols = 128;  // TMEM: CX columns per dy, then 16 of the bias
+constexpr uint32_t kWgCols = 128;  // TMEM columns of an accumulator: CX per dy, then 16 of the bias
+constexpr int kWgRun = 6;        // most tiles summed in one accumulator
 
 constexpr int kWgYRows = kWgKT + 8;  // dY rows staged: the last slot is moved by 7 at most
 // A stage: the dY tile, three x tiles, a tile of ones.
@@ -498,7 +506,7 @@ __host__ __device__ constexpr int wg_smem() {
 }
 
 struct WgHeader {
-    uint64_t full[kWgStages], empty[kWgStages], done;
+    uint64_t full[kWgStages], empty[kWgStages], acc_full[2], acc_empty[2];
     uint32_t tmem_slot;
     int fail;
 };
@@ -508,6 +516,7 @@ struct ConvWgradArgs {
     int W2;          // padded row length
     int chunks;      // tiles per image
     int items;       // tiles of the batch
+    int run;         // tiles summed in one accumulator
 };
 
 // DY covers image rows 1 .. H of the gradient (positions outside read as
@@ -536,7 +545,10 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             dev::mbar_init(&H.full[s], 1);
             dev::mbar_init(&H.empty[s], 1);
         }
-        dev::mbar_init(&H.done, 1);
+        for (int a = 0; a < 2; ++a) {
+            dev::mbar_init(&H.acc_full[a], 1);
+            dev::mbar_init(&H.acc_empty[a], 4);  // one arrival per epilogue warp
+        }
         H.fail = aligned ? 0 : 1;
         if (!aligned) atomicOr(&g_conv_status, 2u);
     }
@@ -546,7 +558,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
     }
     if (warp == 0) {
-        tc::tmem_alloc(&H.tmem_slot, kWgCols);
+        tc::tmem_alloc(&H.tmem_slot, 2 * kWgCols);
         tc::tmem_relinquish();
     }
     tc::fence_proxy_async_smem();
@@ -585,10 +597,12 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         // ---- MMA issue
         constexpr uint32_t id = tc::idesc_bf16_f32(128, 3 * CX + 16, true, true);
         constexpr uint32_t KS_A = 16 * CY * 2, KS_B = 16 * CX * 2;  // 16 positions
-        int k = 0;
+        int k = 0, u = 0, t = 0;  // tile of the range, run u, tile t of the run
         for (int it = i0; it < i1 && !failed(); ++it, ++k) {
-            const int s = k % kWgStages;
-            if (!dev::mbar_wait_bounded(&H.full[s], (uint32_t)((k / kWgStages) & 1), tc::kMmaWaitPolls)) {
+            const int s = k % kWgStages, a = u & 1;
+            if (!dev::mbar_wait_bounded(&H.full[s], (uint32_t)((k / kWgStages) & 1), tc::kMmaWaitPolls) ||
+                (t == 0 &&
+                 !dev::mbar_wait_bounded(&H.acc_empty[a], (uint32_t)(((u >> 1) & 1) ^ 1), tc::kMmaWaitPolls))) {
                 give_up();
                 break;
             }
@@ -599,60 +613,96 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             const uint64_t bd0 = tc::smem_desc_mn<CX>(st + AT, (uint32_t)BT);
 #pragma unroll
             for (int kk = 0; kk < kWgKT / 16; ++kk)
-                tc::mma_bf16(tmem, ad0 + (uint64_t)(kk * KS_A >> 4), bd0 + (uint64_t)(kk * KS_B >> 4), id,
-                             (k | kk) ? 1u : 0u);
+                tc::mma_bf16(tmem + (uint32_t)a * kWgCols, ad0 + (uint64_t)(kk * KS_A >> 4),
+                             bd0 + (uint64_t)(kk * KS_B >> 4), id, (t | kk) ? 1u : 0u);
             tc::mma_commit(&H.empty[s]);
+            if (++t == A.run || it + 1 == i1) {
+                tc::mma_commit(&H.acc_full[a]);
+                t = 0;
+                ++u;
+            }
         }
-        tc::mma_commit(&H.done);
+        // no MMA may still be writing TMEM when it is released; after a wait
+        // that gave up, the run in hand is closed for the epilogue to see it
+        if (t > 0) {
+            tc::mma_commit(&H.acc_full[u & 1]);
+            ++u;
+        }
+        if (u > 0)
+            (void)dev::mbar_wait_bounded(&H.acc_full[(u - 1) & 1], (uint32_t)(((u - 1) >> 1) & 1),
+                                         tc::kMmaWaitPolls);
     } else if (warp >= 2) {
-        // ---- partial sums: row slot * CY + co of the accumulator is tap column
+        // ---- sums: row slot * CY + co of the accumulator is tap column
         // dx = 1 - slot (dY moved by slot - 1 meets x at the opposite offset)
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const int slot = row / CY, co = row % CY;
+        const bool used = quad * 32 < 3 * CY;  // the warp holds rows of the three slots
+        const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
         float* out = A.partial + (size_t)c * (9 * CY * CX + CY);
-        const bool ok = __all_sync(0xFFFFFFFFu, dev::mbar_wait_bounded(&H.done, 0, tc::kMmaWaitPolls)) && !failed();
-        if (!ok) {
-            // a wait gave up: poison this CTA's block so the reduction yields
-            // NaN instead of mixing in what the scratch held before
-            if (lane == 0) give_up();
-            for (int i = tid - 64; i < 9 * CY * CX + CY; i += 128) out[i] = __int_as_float(0x7fc00000);
-        } else {
+        float sum[3 * CX], bias = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 3 * CX; ++j) sum[j] = 0.0f;
+        const int runs = (i1 - i0 + A.run - 1) / A.run;
+#pragma unroll 1
+        for (int u = 0; u < runs; ++u) {
+            const int a = u & 1;
+            const bool full = !failed() && dev::mbar_wait_bounded(&H.acc_full[a], (uint32_t)((u >> 1) & 1),
+                                                                  tc::kMmaWaitPolls);
+            if (!__all_sync(0xFFFFFFFFu, full && !failed())) {
+                if (lane == 0) give_up();
+                break;
+            }
             tc::fence_after_sync();
-            const bool vec = (reinterpret_cast<uintptr_t>(A.partial) & 15u) == 0u;
-            const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
+            if (used) {
+                const uint32_t acc = lanes + (uint32_t)a * kWgCols;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const uint32_t col = (uint32_t)(d * CX);
-#pragma unroll
-                for (int h = 0; h < CX / 16; ++h) {
+                for (int h = 0; h < 3 * CX / 16 + 1; ++h) {
                     uint32_t v[16];
-                    tc::tmem_ld16(lanes + col + (uint32_t)(16 * h), v);
+                    tc::tmem_ld16(acc + (uint32_t)(16 * h), v);
                     tc::tmem_wait_ld();
-                    if (slot < 3) {
-                        float* o = out + ((3 * d + 2 - slot) * CY + co) * CX + 16 * h;
-                        if (vec) {
+                    if (h < 3 * CX / 16) {
 #pragma unroll
-                            for (int j = 0; j < 16; j += 4)
-                                *reinterpret_cast<uint4*>(o + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) o[j] = __uint_as_float(v[j]);
-                        }
+                        for (int j = 0; j < 16; ++j) sum[16 * h + j] += __uint_as_float(v[j]);
+                    } else {
+                        bias += __uint_as_float(v[0]);
                     }
                 }
-                if (d == 1) {
-                    uint32_t v[16];
-                    tc::tmem_ld16(lanes + (uint32_t)(3 * CX), v);
-                    tc::tmem_wait_ld();
-                    if (slot == 1) out[9 * CY * CX + co] = __uint_as_float(v[0]);
+            }
+            // the accumulator is free again
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dev::smem_addr(&H.acc_empty[a]))
+                             : "memory");
+        }
+        // the four warps agree on the outcome
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (failed()) {
+            // a wait gave up: poison this CTA's block so the reduction yields
+            // NaN instead of mixing in what the scratch held before
+            for (int i = tid - 64; i < 9 * CY * CX + CY; i += 128) out[i] = __int_as_float(0x7fc00000);
+        } else if (slot < 3) {
+            const bool vec = (reinterpret_cast<uintptr_t>(A.partial) & 15u) == 0u;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                float* o = out + ((3 * d + 2 - slot) * CY + co) * CX;
+                if (vec) {
+#pragma unroll
+                    for (int j = 0; j < CX; j += 4)
+                        *reinterpret_cast<float4*>(o + j) = make_float4(sum[d * CX + j], sum[d * CX + j + 1],
+                                                                        sum[d * CX + j + 2], sum[d * CX + j + 3]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < CX; ++j) o[j] = sum[d * CX + j];
                 }
             }
+            if (slot == 1) out[9 * CY * CX + co] = bias;
         }
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, kWgCols);
+    if (warp == 0) tc::tmem_dealloc(tmem, 2 * kWgCols);
 }
 
 // dW[co][ci][tap] = sum over CTAs of partial[cta][tap][co][ci]; db[co] likewise.
@@ -906,6 +956,9 @@ int conv3x3_wgrad(const void* x, const void* dy, float* workspace, size_t worksp
     const long long items = (long long)B * a.chunks;
     if (items > 0x7FFFFFFFll) return set_error(PFB_E_ARG, "conv3x3_wgrad: bad shape");
     a.items = (int)items;
+    // a run is no longer than half an image (a whole one below 512 positions)
+    const int n = H * (W + 2), half = n > 448 ? n / (2 * kWgKT) : a.chunks;
+    a.run = half < kWgRun ? half : kWgRun;
     int dev = 0, sms = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
