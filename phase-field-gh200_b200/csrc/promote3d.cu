@@ -165,7 +165,6 @@ __global__ void __launch_bounds__(kThreads3, 2)
     U.k.inter = A.interaction_coeff;
     U.k.dt = A.dt;
     const float* wall = GEO == 2 ? A.wall.values : nullptr;
-    const int strips = E / 4, items = strips * strips;
     UpdateCounts c;
     for (int i = 0; i < PB; ++i) {
         const int dz = d0 + i;
@@ -177,11 +176,8 @@ __global__ void __launch_bounds__(kThreads3, 2)
         const float* p2 = cube_plane(src, L, oz, zs + 1, E);
         const float wallv = GEO == 2 && live ? wall[wz] : 0.0f;
         const bool top_plane = GEO == 1 && live && wz == L.nz - 1;
-        for (int it = tid; it < items; it += kThreads3) {
-            const int x0 = 4 * (it % strips), y0 = 4 * (it / strips);
-            update_item<GEO>(U, p0, p1, p2, x0, y0, sx, sy, live, wz, wallv, top_plane,
-                             dst + ((size_t)dz * E + y0) * E + x0, c);
-        }
+        update_plane<GEO, kThreads3>(U, p0, p1, p2, sx, sy, live, wz, wallv, top_plane,
+                                     dst + (size_t)dz * E * E, c);
     }
     unsigned clip = 0u;
     if ((sx | sy | sz) != 0) clip = clip_check<GEO>(U, src, wall, d0, d1, sx, sy, sz, oz, c, kThreads3);

@@ -250,13 +250,9 @@ __global__ void __launch_bounds__(kThreads3, 2) k_step3d(const __grid_constant__
             const bool live = !H.fail && (unsigned)zs < (unsigned)B && aggregate_z(L, oz, zs, &wz);
             const float wallv = GEO == 2 && live ? wall[wz] : 0.0f;
             const bool top_plane = GEO == 1 && live && wz == L.nz - 1;
-            for (int it = tid; it < items; it += kThreads3) {
-                const int x0 = 4 * (it % strips);
-                const int y0 = 4 * (it / strips);
-                update_item<GEO>(U, ring.slot(base + i), ring.slot(base + i + 1),
-                                 ring.slot(base + i + 2), x0, y0, sx, sy, live, wz, wallv, top_plane,
-                                 dst + ((size_t)dz * B + y0) * B + x0, cnt);
-            }
+            update_plane<GEO, kThreads3>(U, ring.slot(base + i), ring.slot(base + i + 1),
+                                         ring.slot(base + i + 2), sx, sy, live, wz, wallv, top_plane,
+                                         dst + (size_t)dz * B * B, cnt);
             __syncthreads();
             if (!H.fail && issued - base < nreq) {
                 issue_plane(issued, z0 + sz - 1 + (issued - base));

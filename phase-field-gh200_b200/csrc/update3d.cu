@@ -126,8 +126,6 @@ __global__ void __launch_bounds__(kUThreads, 2)
     }
 
     UpdateCounts cnt;
-    const int strips = B / 4;
-    const int items = strips * (B / 4);
     const float* wall = GEO == 2 ? A.wall.values : nullptr;
 
     for (int i = 0; i < PB; ++i) {
@@ -142,13 +140,9 @@ __global__ void __launch_bounds__(kUThreads, 2)
         const bool live = zin && aggregate_z(L, oz, zs, &wz) && !H.abort;
         const float wallv = GEO == 2 && live ? wall[wz] : 0.0f;
         const bool top_plane = GEO == 1 && live && wz == L.nz - 1;
-        for (int it = tid; it < items; it += kUThreads) {
-            const int x0 = 4 * (it % strips);
-            const int y0 = 4 * (it / strips);
-            const uint32_t pix0 = (uint32_t)(((size_t)dz * B + y0) * B + x0);
-            update_item<GEO, T>(U, ring.slot(i), ring.slot(i + 1), ring.slot(i + 2), x0, y0, sx, sy,
-                                live, wz, wallv, top_plane, dst + pix0, cnt, sr, pix0);
-        }
+        const uint32_t pix = (uint32_t)(dz * B * B);
+        update_plane<GEO, kUThreads, T>(U, ring.slot(i), ring.slot(i + 1), ring.slot(i + 2), sx, sy, live,
+                                        wz, wallv, top_plane, dst + pix, cnt, sr, pix);
         __syncthreads();
         // after a timed-out wait nothing more is issued into the ring
         if (!H.abort && i + kURing < nreq) {

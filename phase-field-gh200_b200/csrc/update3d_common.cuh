@@ -161,14 +161,13 @@ struct UpdateCounts {
 __device__ __forceinline__ float2 pair(const float* v) { return make_float2(v[0], v[1]); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, dup2(-1.0f), a); }
 
-// The item below with every test made per voxel: any source offset, columns and
-// rows outside the brick read as zero. Returns its flag counts.
+// The item below read at in-plane offset (sx, sy) of the source, with every test
+// made per voxel: columns and rows outside the brick read as zero.
 template <int GEO, typename T>
-__device__ __noinline__ UpdateCounts update_item_clipped(const UpdateCell U, const T* p0, const T* p1,
-                                                         const T* p2, int x0, int y0, int sx, int sy,
-                                                         int wz, float wallv, bool top_plane, T* orow,
-                                                         uint32_t sr, uint32_t pix0) {
-    UpdateCounts c;
+__device__ __forceinline__ void update_item_moved(const UpdateCell& U, const T* p0, const T* p1,
+                                                  const T* p2, int x0, int y0, int sx, int sy, int wz,
+                                                  float wallv, bool top_plane, T* orow, uint32_t sr,
+                                                  uint32_t pix0, UpdateCounts& c) {
     const int B = U.B;
     const pfb_layout3d& L = U.L;
     const T* pl[3] = {p0, p1, p2};
@@ -252,14 +251,29 @@ __device__ __noinline__ UpdateCounts update_item_clipped(const UpdateCell U, con
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) c.ovf += old_prev[j] > 0xFFFFFFFFu - q_prev[j] ? 1u : 0u;
+}
+
+// The items of a destination plane of a cell shifted in x or y; `out` points at
+// the plane, voxel pix of the brick. One call per plane, out of line: the
+// common case keeps its registers.
+template <int GEO, int NT, typename T>
+__device__ __noinline__ UpdateCounts update_plane_moved(const UpdateCell U, const T* p0, const T* p1,
+                                                        const T* p2, int sx, int sy, int wz, float wallv,
+                                                        bool top_plane, T* out, uint32_t sr, uint32_t pix) {
+    UpdateCounts c;
+    const int strips = U.B / 4;
+    for (int it = threadIdx.x; it < strips * strips; it += NT) {
+        const int x0 = 4 * (it % strips), y0 = 4 * (it / strips);
+        const uint32_t o = (uint32_t)(y0 * U.B + x0);
+        update_item_moved<GEO, T>(U, p0, p1, p2, x0, y0, sx, sy, wz, wallv, top_plane, out + o, sr, pix + o, c);
+    }
     return c;
 }
 
-// One item of destination plane dz: columns x0 .. x0 + 3 of rows
-// y0 .. y0 + 3, read from source plane dz + sz (p1) and its neighbours p0,
-// p2 at in-plane offset (sx, sy); `live` false (source plane outside the
-// brick or the domain) writes zeros. orow points at (dz, y0, x0) of phi_out,
-// voxel pix0 of the brick (16-bit pools: rounding stream sr).
+// One item of a destination plane of an unshifted cell: columns x0 .. x0 + 3 of
+// rows y0 .. y0 + 3, read from source plane p1 and its neighbours p0, p2. orow
+// points at (y0, x0) of the plane in phi_out, voxel pix0 of the brick (16-bit
+// pools: rounding stream sr).
 // GEO: 0 periodic, 1 substrate slab, 2 hard-wall channel.
 //
 // The sweep is bound by the instructions a voxel takes, so the flag tests are
@@ -270,45 +284,25 @@ __device__ __noinline__ UpdateCounts update_item_clipped(const UpdateCell U, con
 // the update and the measurement below the same rule take 2.87 instead of 3.41
 // ms for two steps of 512 cells (B = 64, periodic), 2.17 instead of 2.87 ms for
 // 187 cells of a slab (B = 80). The Laplacian stays scalar: packing the middle
-// column of taps as well measured 1 % slower (more spills). Items whose source
-// columns or rows leave the brick (shifted cells) take the per-voxel form above.
+// column of taps as well measured 1 % slower (more spills).
 template <int GEO, typename T = float>
 __device__ __forceinline__ void update_item(const UpdateCell& U, const T* p0, const T* p1,
-                                            const T* p2, int x0, int y0, int sx, int sy,
-                                            bool live, int wz, float wallv, bool top_plane,
-                                            T* orow, UpdateCounts& c, uint32_t sr = 0u,
-                                            uint32_t pix0 = 0u) {
+                                            const T* p2, int x0, int y0, int wz, float wallv,
+                                            bool top_plane, T* orow, UpdateCounts& c, uint32_t sr,
+                                            uint32_t pix0) {
     const int B = U.B;
     const pfb_layout3d& L = U.L;
-    if (!live) {
-        const float z[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint16_t zb[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int r = 0; r < 4; ++r) phi_st4(orow + r * B, z, zb);
-        return;
-    }
-    const int xs0 = x0 + sx, ys0 = y0 + sy;
-    if ((xs0 & 3) != 0 || xs0 < 0 || xs0 + 4 > B || ys0 < 0 || ys0 + 4 > B) {
-        const UpdateCounts d = update_item_clipped<GEO, T>(U, p0, p1, p2, x0, y0, sx, sy, wz, wallv,
-                                                           top_plane, orow, sr, pix0);
-        c.nf += d.nf;
-        c.neg += d.neg;
-        c.top += d.top;
-        c.clamp += d.clamp;
-        c.ovf += d.ovf;
-        return;
-    }
     const T* pl[3] = {p0, p1, p2};
     float w[3][3][6];
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-        row6v(pl[p], B, ys0 - 1, xs0, true, w[p][0]);
-        row6v(pl[p], B, ys0, xs0, true, w[p][1]);
+        row6v(pl[p], B, y0 - 1, x0, true, w[p][0]);
+        row6v(pl[p], B, y0, x0, true, w[p][1]);
     }
     int wxj[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) wxj[j] = wrap_offset(U.ox, xs0 + j, L.nx);
-    int wy = wrap_offset(U.oy, ys0, L.ny);
+    for (int j = 0; j < 4; ++j) wxj[j] = wrap_offset(U.ox, x0 + j, L.nx);
+    int wy = wrap_offset(U.oy, y0, L.ny);
     const bool has_out = U.S_out != nullptr;
     const uint32_t* s_in = U.S_in + s_index(L, 0, 0, wz);
     uint32_t* s_out = U.S_out + (has_out ? s_index(L, 0, 0, wz) : 0);
@@ -324,7 +318,7 @@ __device__ __forceinline__ void update_item(const UpdateCell& U, const T* p0, co
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
 #pragma unroll
-        for (int p = 0; p < 3; ++p) row6v(pl[p], B, ys0 + r + 1, xs0, true, w[p][(r + 2) % 3]);
+        for (int p = 0; p < 3; ++p) row6v(pl[p], B, y0 + r + 1, x0, true, w[p][(r + 2) % 3]);
         uint32_t agg[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) agg[j] = agg_next[j];
@@ -404,6 +398,40 @@ __device__ __forceinline__ void update_item(const UpdateCell& U, const T* p0, co
     if (pending) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) c.ovf += old_prev[j] > 0xFFFFFFFFu - q_prev[j] ? 1u : 0u;
+    }
+}
+
+// Destination plane `out` (voxel pix of the brick) of a cell, read from source
+// plane p1 and its neighbours at in-plane offset (sx, sy); `live` false (source
+// plane outside the brick or the domain) writes zeros. Every thread of a CTA of
+// NT. A cell shifted in x or y takes the per-voxel form for all its items: chosen
+// item by item, only where the source leaves the brick, both forms ran in the
+// warps along the brick's edge (300 cells of the channel, B = 40, all shifted by
+// one row: 738 us against 406; by four columns 968 against 731).
+template <int GEO, int NT, typename T = float>
+__device__ __forceinline__ void update_plane(const UpdateCell& U, const T* p0, const T* p1, const T* p2,
+                                             int sx, int sy, bool live, int wz, float wallv,
+                                             bool top_plane, T* out, UpdateCounts& c, uint32_t sr = 0u,
+                                             uint32_t pix = 0u) {
+    const int strips = U.B / 4, items = strips * strips;
+    if (live && (sx | sy) == 0) {
+        for (int it = threadIdx.x; it < items; it += NT) {
+            const int x0 = 4 * (it % strips), y0 = 4 * (it / strips);
+            const uint32_t o = (uint32_t)(y0 * U.B + x0);
+            update_item<GEO, T>(U, p0, p1, p2, x0, y0, wz, wallv, top_plane, out + o, c, sr, pix + o);
+        }
+    } else if (live) {
+        const UpdateCounts d =
+            update_plane_moved<GEO, NT, T>(U, p0, p1, p2, sx, sy, wz, wallv, top_plane, out, sr, pix);
+        c.nf += d.nf;
+        c.neg += d.neg;
+        c.top += d.top;
+        c.clamp += d.clamp;
+        c.ovf += d.ovf;
+    } else {
+        const float z[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint16_t zb[4] = {0, 0, 0, 0};
+        for (int q = 4 * (int)threadIdx.x; q < U.B * U.B; q += 4 * NT) phi_st4(out + q, z, zb);
     }
 }
 
