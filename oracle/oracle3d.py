@@ -52,6 +52,9 @@ def olib() -> C.CDLL:
         L.oracle3d_measure.restype = None
         L.oracle3d_scatter.argtypes = [I, P, P, P, P, C.POINTER(Layout3D), I, I]
         L.oracle3d_scatter.restype = None
+        L.oracle3d_update.argtypes = [P, P, P, P, P, P, C.POINTER(Layout3D), I, I, P, D, D, D, D,
+                                      D, I]
+        L.oracle3d_update.restype = None
         L.oracle3d_q32.argtypes = [C.c_float]
         L.oracle3d_q32.restype = C.c_uint32
         _O = L

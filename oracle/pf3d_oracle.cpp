@@ -635,6 +635,23 @@ void oracle3d_measure(int f64, const void* phi, const uint32_t* S, pfb_cell3d* c
     if (motion_too) motion(cells, gflags, m, f64 != 0, 60.0 * kappa / (xi * lambda * lambda), vel);
 }
 
+// The update alone (binary32): cells' own velocities, pending shifts and volumes;
+// phi_out written, S_out added to, flags raised.
+void oracle3d_update(const float* phi_in, float* phi_out, const uint32_t* S_in, uint32_t* S_out,
+                     pfb_cell3d* cells, uint32_t* gflags, const pfb_layout3d* L, int N, int B,
+                     const float* wall, double dt, double V0, double volume_scale, double bulk_scale,
+                     double inter, int threads) {
+    set_threads(threads);
+    std::vector<double> vel((size_t)3 * N);
+    for (int n = 0; n < N; ++n) {
+        vel[3 * n] = cells[n].velocity_x;
+        vel[3 * n + 1] = cells[n].velocity_y;
+        vel[3 * n + 2] = cells[n].velocity_z;
+    }
+    UArgs u{L, N, B, wall, dt, V0, volume_scale, bulk_scale, inter};
+    update(phi_in, phi_out, S_in, S_out, cells, gflags, u, vel);
+}
+
 void oracle3d_scatter(int f64, const void* phi, pfb_cell3d* cells, uint32_t* S, uint32_t* gflags,
                       const pfb_layout3d* L, int N, int B) {
     if (f64)
