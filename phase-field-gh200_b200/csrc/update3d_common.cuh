@@ -33,29 +33,6 @@ __device__ __forceinline__ bool fatal3(const pfb_cell3d* cell, const uint32_t* g
     return false;
 }
 
-// The 27-point Laplacian and centred gradients of column j (0..3) of the
-// window w[plane][row][col], plane/row 0 = -1 offset: weights and the z, y, x
-// summation order of the reference's stencil27_at.
-__device__ __forceinline__ void stencil27w(const float (&w)[3][3][6], int j, float& lap,
-                                           float& gx, float& gy, float& gz) {
-    float acc = (float)kWCentre * w[1][1][j + 1];
-#pragma unroll
-    for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-            for (int dx = 0; dx < 3; ++dx) {
-                const int d = (dz != 1) + (dy != 1) + (dx != 1);
-                if (d == 0) continue;
-                const int wgt = d == 1 ? kWFace : d == 2 ? kWEdge : kWCorner;
-                acc += (float)wgt * w[dz][dy][j + dx];
-            }
-    lap = acc * (float)(1.0 / 30.0);
-    gx = 0.5f * (w[1][1][j + 2] - w[1][1][j]);
-    gy = 0.5f * (w[1][2][j + 1] - w[1][0][j + 1]);
-    gz = 0.5f * (w[2][1][j + 1] - w[0][1][j + 1]);
-}
-
 // Six source values of one row, columns xs0 - 1 .. xs0 + 4 (zero outside the
 // brick or when the row is outside it); the alignment decision is taken once
 // per strip.
@@ -80,9 +57,11 @@ __device__ __forceinline__ void row6v(const T* plane, int B, int ys, int xs0, bo
     }
 }
 
-// stencil27w over a window whose rows rotate through slots: row offset -1,
-// 0, +1 of every plane live in slots s0, s1, s2. The sum's rounding is written
-// out (left as + and *, pairs of columns were compiled to other roundings).
+// The 27-point Laplacian of column j (0..3) of the window w[plane][row][col],
+// plane 0 = -1 offset: weights and the z, y, x summation order of the reference's
+// stencil27_at. The window's rows rotate through slots: row offset -1, 0, +1 of
+// every plane live in slots s0, s1, s2. The sum's rounding is written out (left
+// as + and *, pairs of columns were compiled to other roundings).
 __device__ __forceinline__ float laplace27r(const float (&w)[3][3][6], int s0, int s1, int s2, int j) {
     const int sl[3] = {s0, s1, s2};
     float acc = __fmul_rn((float)kWCentre, w[1][s1][j + 1]);
@@ -100,6 +79,7 @@ __device__ __forceinline__ float laplace27r(const float (&w)[3][3][6], int s0, i
     return __fmul_rn(acc, (float)(1.0 / 30.0));
 }
 
+// The same with the centred gradients.
 __device__ __forceinline__ void stencil27r(const float (&w)[3][3][6], int s0, int s1, int s2,
                                            int j, float& lap, float& gx, float& gy, float& gz) {
     lap = laplace27r(w, s0, s1, s2, j);
@@ -499,7 +479,7 @@ __device__ __forceinline__ unsigned clip_check(const UpdateCell& U, const T* src
 #pragma unroll
                 for (int cc = 0; cc < 3; ++cc) wv[p][r][cc] = f(x + cc - 1, y + r - 1, z + p - 1);
         float lap, gx, gy, gz;
-        stencil27w(wv, 0, lap, gx, gy, gz);
+        stencil27r(wv, 0, 1, 2, 0, lap, gx, gy, gz);
         if (cv == 0.0f && lap == 0.0f && gx == 0.0f && gy == 0.0f && gz == 0.0f) continue;
         const size_t si = s_index(L, wrap_offset(U.ox, x, L.nx), wrap_offset(U.oy, y, L.ny), wz);
         const uint32_t agg = U.S_in[si];
