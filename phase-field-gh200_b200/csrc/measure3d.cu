@@ -227,11 +227,15 @@ static int measure_launch_k(const pfb_measure_args3d& A, int count, cudaStream_t
 }
 
 // Parts to cut each of `cells` cells into: as many, from `least` to `most`, as
-// still run in one wave at two CTAs per SM. A part stages two halo planes more
-// than it owns, so cells that fill the SMs stay at `least`. 12 channel cells
-// (B = 64), four steps: 718 us at 4 parts, 333 us with this rule (clusters of 8,
-// 24 update parts; 363 us at 16); 512 cells keep 4.
-int parts_in_one_wave3d(int cells, int least, int most) {
+// there are two CTAs for every SM. A part stages two halo planes more than it
+// owns, so cells that fill the SMs stay at `least`. 12 channel cells (B = 64),
+// four steps: 718 us at 4 parts, 333 us with this rule (clusters of 8, 24 update
+// parts; 363 us at 16); 512 cells keep 4. Where the plane ring of a binary32
+// brick leaves room for one CTA per SM (the update from B = 80, the measurement
+// from 88) these parts run in two waves, which still beats as many as run in
+// one: a step of B = 80 takes 268 us at 30 cells and 388 us at 38, with one CTA
+// for every SM 288 and 489; at 12 cells 169 and 160.
+int parts_per_cell3d(int cells, int least, int most) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -242,7 +246,7 @@ int parts_in_one_wave3d(int cells, int least, int most) {
 
 // The measurement's cluster size. 4 where the cells fill the SMs (fewer halo
 // planes and folds); 8 where a system of few cells would leave SMs idle.
-int measure3d_cluster(int cells) { return parts_in_one_wave3d(cells, 4, 8) == 8 ? 8 : 4; }
+int measure3d_cluster(int cells) { return parts_per_cell3d(cells, 4, 8) == 8 ? 8 : 4; }
 
 template <typename T>
 static int measure_launch_t(const pfb_measure_args3d& A, int count, cudaStream_t stream) {

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kUThreads, 2)
 // Host side
 // ---------------------------------------------------------------------------
 int geometry_ok3(int B, const pfb_layout3d& L);
-int parts_in_one_wave3d(int cells, int least, int most);
+int parts_per_cell3d(int cells, int least, int most);
 
 size_t update3d_smem(int B, int bytes = 4) {
     return (size_t)kUHeader + (size_t)kURing * (size_t)B * B * bytes;
@@ -223,8 +223,9 @@ static int update_launch(const pfb_update_args3d& A, int out_by_slot, int storag
     if (smem > 227 * 1024) return set_error(PFB_E_CONFIG, "brick edge too large for the plane ring");
     // a few cells are cut into more parts (of 2 planes at least: each part
     // stages two planes more than it updates) so that the SMs are not idle;
-    // the result does not depend on the cut
-    const int parts = parts_in_one_wave3d(count, kUCtasPerCell, A.B / 2);
+    // without a fatal flag the result does not depend on the cut (a CTA that
+    // starts after the flag was raised keeps its planes' accepted field)
+    const int parts = parts_per_cell3d(count, kUCtasPerCell, A.B / 2);
     const dim3 grid((unsigned)(count * parts));
     cudaError_t e;
     if (storage == kStoreF16)
