@@ -22,6 +22,8 @@ constexpr int kDefaultCluster = 2;
 int step2d_smem_bytes(int cluster);
 // Systems r = 0..R-1 in one launch: d_args[r] (device) is served by CTAs
 // [d_block_start[r], d_block_start[r+1]) (R+1 entries, multiples of cluster).
+// CTAs of a step that the current device runs at once (0: no device).
+int step2d_wave(int cluster);
 int step2d_read_status(unsigned* out, int clear);
 int init2d_read_status(unsigned* out, int clear);
 // variant: 0 = default, 1 = one thread-block cluster per cell
@@ -52,7 +54,9 @@ int step2d_launch_binned(const pfb_step_args2d* a, int cluster, int storage, con
 int step2d_settle_bins(const BinArgs& B, const void* phi, int storage, int N, int L,
                        unsigned long long step, uint32_t* flags, cudaStream_t stream);
 // R systems in one launch, and the settling of their last launch's bounds
-// (d_next: the arguments of their next step). Tables in device memory.
+// (d_next: the arguments of their next step). Tables in device memory. Without
+// bounds (d_bins null) the launch scatters with returns and leaves nothing to
+// settle.
 int step2d_launch_batch(const pfb_step_args2d* d_args, const BinArgs* d_bins,
                         const int* d_block_start, int R, int total_blocks, int cluster, int storage,
                         cudaStream_t stream);

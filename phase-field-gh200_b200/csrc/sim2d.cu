@@ -1014,16 +1014,17 @@ struct pfb_ens2d {
     int* d_start = nullptr;             // R + 1 block offsets
     int total_blocks = 0;
     bool tables_ready = false;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
+    int wave = 0;  // CTAs that run at once
+    // six-step graphs, by scatter (returning, under bounds)
+    cudaGraphExec_t graph_exec[2] = {};
     // trajectory recording: sources of the batched pack (system order), the
     // ring header, a device frame for pageable rings, record graphs
-    // [every - 1][phase] as pfb_sim2d's
+    // [scatter][every - 1][phase] as pfb_sim2d's
     TrajSource2D* d_src = nullptr;
     TrajRing2D* d_ring = nullptr;
     pfb_traj_cell2d* d_frame = nullptr;
     int total_cells = 0;
-    cudaGraphExec_t rec_exec[6][6] = {};
+    cudaGraphExec_t rec_exec[2][6][6] = {};
 
     ~pfb_ens2d() {
         drop_graph();
@@ -1040,15 +1041,25 @@ struct pfb_ens2d {
     int R() const { return (int)sims.size(); }
 
     void drop_graph() {
-        if (graph_exec) cudaGraphExecDestroy(graph_exec);
-        if (graph) cudaGraphDestroy(graph);
-        graph_exec = nullptr;
-        graph = nullptr;
-        for (auto& row : rec_exec)
-            for (cudaGraphExec_t& e : row) {
-                if (e) cudaGraphExecDestroy(e);
-                e = nullptr;
-            }
+        auto drop = [](cudaGraphExec_t& e) {
+            if (e) cudaGraphExecDestroy(e);
+            e = nullptr;
+        };
+        for (cudaGraphExec_t& e : graph_exec) drop(e);
+        for (auto& scatter : rec_exec)
+            for (auto& row : scatter)
+                for (cudaGraphExec_t& e : row) drop(e);
+    }
+
+    // Whether an advance of `steps` scatters without returns, under the bin
+    // bounds (same bits either way). That saves about 2.2 us a step for every
+    // wave of CTAs beyond the first (1.7 us at 256 cells in clusters of 2, 5.4
+    // at 512, nothing where one wave holds the batch) and costs the 4.1 us of
+    // the launch that settles the bounds at the end. One step of 2 systems of
+    // 16 cells: 24.9 us with returns, 29.1 under bounds; of 32 systems of 64
+    // cells 350 and 337.
+    bool bounds_pay(long long steps) const {
+        return total_blocks > wave && steps * (total_blocks - wave) >= 2ll * wave;
     }
 
     // The pack sources in system order (buffers are fixed for the life of
@@ -1073,11 +1084,11 @@ struct pfb_ens2d {
 
     int pack() { return pack_traj2d_ring_batch(d_src, R(), total_cells, d_ring, stream); }
 
-    int build_record_graph(int every, int phase) {
+    int build_record_graph(bool bounds, int every, int phase) {
         PFB_CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         int rc = PFB_OK;
         for (int s = 0; s < 6 && rc == PFB_OK; ++s) {
-            rc = launch_slot(s);
+            rc = launch_slot(s, bounds);
             if (rc == PFB_OK && (phase + s + 1) % every == 0) rc = pack();
         }
         cudaGraph_t g = nullptr;
@@ -1087,7 +1098,7 @@ struct pfb_ens2d {
             return rc;
         }
         PFB_CU(e, "end capture");
-        const cudaError_t ie = cudaGraphInstantiateWithFlags(&rec_exec[every - 1][phase], g, 0);
+        const cudaError_t ie = cudaGraphInstantiateWithFlags(&rec_exec[bounds][every - 1][phase], g, 0);
         cudaGraphDestroy(g);
         PFB_CU(ie, "graph instantiate");
         return PFB_OK;
@@ -1112,29 +1123,30 @@ struct pfb_ens2d {
         (void)cudaGetLastError();  // an unregistered pointer is not an error here
         if (const int rc = ring_begin2d(d_ring, dring ? dring : d_frame, dring ? frames : 1, stream)) return rc;
         const bool rec_graph = dring && 6 % every == 0;
+        const bool bounds = bounds_pay(steps);
         long long done = 0, k = 0;
         while (done < steps) {
             const bool aligned = steps_done % 6 == 0 && steps - done >= 6;
             if (rec_graph && aligned) {
                 const int phase = (int)(done % every);
-                if (!rec_exec[every - 1][phase]) {
-                    if (const int rc = build_record_graph(every, phase)) return rc;
+                if (!rec_exec[bounds][every - 1][phase]) {
+                    if (const int rc = build_record_graph(bounds, every, phase)) return rc;
                 }
-                PFB_CU(cudaGraphLaunch(rec_exec[every - 1][phase], stream), "graph launch");
+                PFB_CU(cudaGraphLaunch(rec_exec[bounds][every - 1][phase], stream), "graph launch");
                 steps_done += 6;
                 done += 6;
                 continue;
             }
             const long long due = (done / every + 1) * every;
             if (aligned && due >= done + 6) {
-                if (!graph_exec) {
-                    if (const int rc = build_graph()) return rc;
+                if (!graph_exec[bounds]) {
+                    if (const int rc = build_graph(bounds)) return rc;
                 }
-                PFB_CU(cudaGraphLaunch(graph_exec, stream), "graph launch");
+                PFB_CU(cudaGraphLaunch(graph_exec[bounds], stream), "graph launch");
                 steps_done += 6;
                 done += 6;
             } else {
-                if (const int rc = launch_slot((int)(steps_done % 6))) return rc;
+                if (const int rc = launch_slot((int)(steps_done % 6), bounds)) return rc;
                 steps_done += 1;
                 done += 1;
             }
@@ -1148,7 +1160,7 @@ struct pfb_ens2d {
             }
         }
         for (pfb_sim2d* s : sims) s->steps_done = steps_done;
-        return steps > 0 ? settle() : PFB_OK;
+        return bounds ? settle() : PFB_OK;
     }
 
     // Argument tables for the six slots and the CTA offsets for `cluster`.
@@ -1165,6 +1177,7 @@ struct pfb_ens2d {
             start[(size_t)i + 1] = start[(size_t)i] + s->N * cluster;
         }
         total_blocks = start[(size_t)R_];
+        wave = step2d_wave(cluster);
         if (!d_args) PFB_CU(cudaMalloc(&d_args, h.size() * sizeof(pfb_step_args2d)), "alloc args");
         if (!d_bins) PFB_CU(cudaMalloc(&d_bins, bins.size() * sizeof(BinArgs)), "alloc bin table");
         if (!d_start) PFB_CU(cudaMalloc(&d_start, start.size() * sizeof(int)), "alloc offsets");
@@ -1179,22 +1192,21 @@ struct pfb_ens2d {
         return PFB_OK;
     }
 
-    int launch_slot(int slot) {
-        return step2d_launch_batch(d_args + (size_t)slot * R(), d_bins, d_start, R(), total_blocks,
-                                   cluster, storage, stream);
+    int launch_slot(int slot, bool bounds) {
+        return step2d_launch_batch(d_args + (size_t)slot * R(), bounds ? d_bins : nullptr, d_start, R(),
+                                   total_blocks, cluster, storage, stream);
     }
 
-    // Settle the bounds of the last batch launch: the flags are final when an
-    // advance ends, and every other path finds both sets clear.
+    // Settle the bounds of the last launch under them: the flags are final
+    // when an advance ends, and every other path finds both sets clear.
     int settle() {
         return step2d_settle_batch(d_args + (size_t)(steps_done % 6) * R(), d_bins, R(), storage, stream);
     }
 
-    int build_graph() {
-        drop_graph();
+    int build_graph(bool bounds) {
         PFB_CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         int rc = PFB_OK;
-        for (int s = 0; s < 6 && rc == PFB_OK; ++s) rc = launch_slot(s);
+        for (int s = 0; s < 6 && rc == PFB_OK; ++s) rc = launch_slot(s, bounds);
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(stream, &g);
         if (rc != PFB_OK) {
@@ -1202,8 +1214,9 @@ struct pfb_ens2d {
             return rc;
         }
         PFB_CU(e, "end capture");
-        graph = g;
-        PFB_CU(cudaGraphInstantiateWithFlags(&graph_exec, graph, 0), "graph instantiate");
+        const cudaError_t ie = cudaGraphInstantiateWithFlags(&graph_exec[bounds], g, 0);
+        cudaGraphDestroy(g);
+        PFB_CU(ie, "graph instantiate");
         return PFB_OK;
     }
 
@@ -1212,25 +1225,25 @@ struct pfb_ens2d {
             const int rc = build_tables();
             if (rc) return rc;
         }
-        const bool ran = steps > 0;
+        const bool bounds = bounds_pay(steps);
         while (steps > 0) {
             if (steps_done % 6 == 0 && steps >= 6) {
-                if (!graph_exec) {
-                    const int rc = build_graph();
+                if (!graph_exec[bounds]) {
+                    const int rc = build_graph(bounds);
                     if (rc) return rc;
                 }
-                PFB_CU(cudaGraphLaunch(graph_exec, stream), "graph launch");
+                PFB_CU(cudaGraphLaunch(graph_exec[bounds], stream), "graph launch");
                 steps_done += 6;
                 steps -= 6;
             } else {
-                const int rc = launch_slot((int)(steps_done % 6));
+                const int rc = launch_slot((int)(steps_done % 6), bounds);
                 if (rc) return rc;
                 steps_done += 1;
                 steps -= 1;
             }
         }
         for (pfb_sim2d* s : sims) s->steps_done = steps_done;
-        return ran ? settle() : PFB_OK;
+        return bounds ? settle() : PFB_OK;
     }
 
     // The same steps with one launch per system (the replicas-one-at-a-time

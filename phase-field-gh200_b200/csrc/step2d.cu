@@ -882,15 +882,15 @@ __global__ void __launch_bounds__(kThreads, min_blocks(K))
 // Many independent systems in one launch: system r is served by CTAs
 // [block_start[r], block_start[r+1]) (multiples of K, so clusters never
 // straddle systems); its arguments are copied into shared memory. All
-// systems of one launch share the pool storage type T. The scatter is the
+// systems of one launch share the pool storage type T. BINS: the scatter is the
 // non-returning one under each system's own bin bounds.
-template <int K, typename T = float>
+template <int K, typename T, bool BINS>
 __global__ void __launch_bounds__(kThreads, min_blocks(K))
     k_step2d_batch(const pfb_step_args2d* __restrict__ args, const BinArgs* __restrict__ bins,
                    const int* __restrict__ block_start, int R) {
     extern __shared__ __align__(128) char smem[];
     __shared__ __align__(16) pfb_step_args2d sA;
-    __shared__ __align__(16) BinArgs sB;
+    __shared__ __align__(16) BinArgs sB;  // BINS
     const int b = (int)blockIdx.x;
     int lo = 0, hi = R - 1;  // last r with block_start[r] <= b
     while (lo < hi) {
@@ -906,12 +906,12 @@ __global__ void __launch_bounds__(kThreads, min_blocks(K))
     uint64_t* dstw = reinterpret_cast<uint64_t*>(&sA);
     if (threadIdx.x < sizeof(pfb_step_args2d) / 8) dstw[threadIdx.x] = __ldg(srcw + threadIdx.x);
     static_assert(sizeof(BinArgs) % 8 == 0, "bin record copy");
-    if (threadIdx.x < sizeof(BinArgs) / 8)
+    if (BINS && threadIdx.x < sizeof(BinArgs) / 8)
         reinterpret_cast<uint64_t*>(&sB)[threadIdx.x] =
             __ldg(reinterpret_cast<const uint64_t*>(bins + r) + threadIdx.x);
     __syncthreads();
     const int b0 = __ldg(block_start + r);
-    step_body<K, T, PFB_VELOCITY_DISABLED, true>(sA, b - b0, __ldg(block_start + r + 1) - b0, smem, sB);
+    step_body<K, T, PFB_VELOCITY_DISABLED, BINS>(sA, b - b0, __ldg(block_start + r + 1) - b0, smem, sB);
 }
 
 // ---------------------------------------------------------------------------
@@ -931,11 +931,13 @@ static cudaError_t configure_pool() {
     e = cudaFuncSetAttribute(k_step2d<K, T, PFB_VELOCITY_DISABLED, true>,
                              cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_step2d_batch<K, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             step_smem_bytes(K));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_step2d_batch<K, T>,
-                                cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    for (auto batch : {k_step2d_batch<K, T, false>, k_step2d_batch<K, T, true>}) {
+        e = cudaFuncSetAttribute(batch, cudaFuncAttributeMaxDynamicSharedMemorySize, step_smem_bytes(K));
+        if (e != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(batch, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 template <int K, int OBS>
@@ -1186,7 +1188,7 @@ int step2d_launch_variant(const pfb_step_args2d* a, int cluster, int variant,
     return step2d_launch_storage(a, cluster, variant, kStoreF32, stream);
 }
 
-template <int K, typename T = float>
+template <int K, typename T>
 static cudaError_t launch_batch_k(const pfb_step_args2d* args, const BinArgs* bins,
                                   const int* block_start, int R, int total_blocks,
                                   cudaStream_t stream) {
@@ -1202,13 +1204,14 @@ static cudaError_t launch_batch_k(const pfb_step_args2d* args, const BinArgs* bi
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_step2d_batch<K, T>, args, bins, block_start, R);
+    return bins ? cudaLaunchKernelEx(&cfg, k_step2d_batch<K, T, true>, args, bins, block_start, R)
+                : cudaLaunchKernelEx(&cfg, k_step2d_batch<K, T, false>, args, bins, block_start, R);
 }
 
 int step2d_launch_batch(const pfb_step_args2d* d_args, const BinArgs* d_bins,
                         const int* d_block_start, int R, int total_blocks, int cluster, int storage,
                         cudaStream_t stream) {
-    if (!d_args || !d_bins || !d_block_start || R <= 0 || total_blocks < 0)
+    if (!d_args || !d_block_start || R <= 0 || total_blocks < 0)
         return set_error(PFB_E_ARG, "invalid batch arguments");
     if (cluster == 0) cluster = kDefaultCluster;
     if (cluster != 2 && cluster != 4 && cluster != 8)
@@ -1229,11 +1232,19 @@ int step2d_launch_batch(const pfb_step_args2d* d_args, const BinArgs* d_bins,
                 ? launch_batch_k<2, __nv_bfloat16>(d_args, d_bins, d_block_start, R, total_blocks, stream)
                 : launch_batch_k<4, __nv_bfloat16>(d_args, d_bins, d_block_start, R, total_blocks, stream);
     else
-        e = cluster == 2   ? launch_batch_k<2>(d_args, d_bins, d_block_start, R, total_blocks, stream)
-            : cluster == 4 ? launch_batch_k<4>(d_args, d_bins, d_block_start, R, total_blocks, stream)
-                           : launch_batch_k<8>(d_args, d_bins, d_block_start, R, total_blocks, stream);
+        e = cluster == 2   ? launch_batch_k<2, float>(d_args, d_bins, d_block_start, R, total_blocks, stream)
+            : cluster == 4 ? launch_batch_k<4, float>(d_args, d_bins, d_block_start, R, total_blocks, stream)
+                           : launch_batch_k<8, float>(d_args, d_bins, d_block_start, R, total_blocks, stream);
     if (e != cudaSuccess) return set_error(PFB_E_CUDA, "batch launch: %s", cudaGetErrorString(e));
     return PFB_OK;
+}
+
+int step2d_wave(int cluster) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return min_blocks(cluster) * sms;
 }
 
 int step2d_launch(const pfb_step_args2d* a, int cluster, cudaStream_t stream) {
