@@ -250,10 +250,10 @@ __device__ __noinline__ UpdateCounts update_plane_moved(const UpdateCell U, cons
     return c;
 }
 
-// One item of a destination plane of an unshifted cell: columns x0 .. x0 + 3 of
-// rows y0 .. y0 + 3, read from source plane p1 and its neighbours p0, p2. orow
-// points at (y0, x0) of the plane in phi_out, voxel pix0 of the brick (16-bit
-// pools: rounding stream sr).
+// One item of a destination plane of a cell not shifted in x or y: columns xs0 ..
+// xs0 + 3 of rows ys0 .. ys0 + 3, read from source plane p1 and its neighbours
+// p0, p2. orow points at (ys0, xs0) of the plane in phi_out, voxel pix0 of the
+// brick (16-bit pools: rounding stream sr).
 // GEO: 0 periodic, 1 substrate slab, 2 hard-wall channel.
 //
 // The sweep is bound by the instructions a voxel takes, so the flag tests are
@@ -267,7 +267,7 @@ __device__ __noinline__ UpdateCounts update_plane_moved(const UpdateCell U, cons
 // column of taps as well measured 1 % slower (more spills).
 template <int GEO, typename T = float>
 __device__ __forceinline__ void update_item(const UpdateCell& U, const T* p0, const T* p1,
-                                            const T* p2, int x0, int y0, int wz, float wallv,
+                                            const T* p2, int xs0, int ys0, int wz, float wallv,
                                             bool top_plane, T* orow, UpdateCounts& c, uint32_t sr,
                                             uint32_t pix0) {
     const int B = U.B;
@@ -276,13 +276,13 @@ __device__ __forceinline__ void update_item(const UpdateCell& U, const T* p0, co
     float w[3][3][6];
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-        row6v(pl[p], B, y0 - 1, x0, true, w[p][0]);
-        row6v(pl[p], B, y0, x0, true, w[p][1]);
+        row6v(pl[p], B, ys0 - 1, xs0, true, w[p][0]);
+        row6v(pl[p], B, ys0, xs0, true, w[p][1]);
     }
     int wxj[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) wxj[j] = wrap_offset(U.ox, x0 + j, L.nx);
-    int wy = wrap_offset(U.oy, y0, L.ny);
+    for (int j = 0; j < 4; ++j) wxj[j] = wrap_offset(U.ox, xs0 + j, L.nx);
+    int wy = wrap_offset(U.oy, ys0, L.ny);
     const bool has_out = U.S_out != nullptr;
     const uint32_t* s_in = U.S_in + s_index(L, 0, 0, wz);
     uint32_t* s_out = U.S_out + (has_out ? s_index(L, 0, 0, wz) : 0);
@@ -298,7 +298,7 @@ __device__ __forceinline__ void update_item(const UpdateCell& U, const T* p0, co
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
 #pragma unroll
-        for (int p = 0; p < 3; ++p) row6v(pl[p], B, y0 + r + 1, x0, true, w[p][(r + 2) % 3]);
+        for (int p = 0; p < 3; ++p) row6v(pl[p], B, ys0 + r + 1, xs0, true, w[p][(r + 2) % 3]);
         uint32_t agg[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) agg[j] = agg_next[j];
@@ -388,6 +388,10 @@ __device__ __forceinline__ void update_item(const UpdateCell& U, const T* p0, co
 // item by item, only where the source leaves the brick, both forms ran in the
 // warps along the brick's edge (300 cells of the channel, B = 40, all shifted by
 // one row: 738 us against 406; by four columns 968 against 731).
+//
+// The other cells' offset is zero; adding it in the bounded geometries alone is
+// for the register allocation: the update of 187 slab cells takes 561 us with it
+// and 582 without, that of 512 periodic cells 846 and 835.
 template <int GEO, int NT, typename T = float>
 __device__ __forceinline__ void update_plane(const UpdateCell& U, const T* p0, const T* p1, const T* p2,
                                              int sx, int sy, bool live, int wz, float wallv,
@@ -398,7 +402,8 @@ __device__ __forceinline__ void update_plane(const UpdateCell& U, const T* p0, c
         for (int it = threadIdx.x; it < items; it += NT) {
             const int x0 = 4 * (it % strips), y0 = 4 * (it / strips);
             const uint32_t o = (uint32_t)(y0 * U.B + x0);
-            update_item<GEO, T>(U, p0, p1, p2, x0, y0, wz, wallv, top_plane, out + o, c, sr, pix + o);
+            update_item<GEO, T>(U, p0, p1, p2, GEO ? x0 + sx : x0, GEO ? y0 + sy : y0, wz, wallv,
+                                top_plane, out + o, c, sr, pix + o);
         }
     } else if (live) {
         const UpdateCounts d =
