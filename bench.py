@@ -615,7 +615,7 @@ def profile_conv_layers(local, batch=512, repeats=20):
     the median CUDA-event time of one pfb_conv3x3_forward (bias, ReLU,
     bfloat16 output) over `repeats` launches after 3 warm-up ones, L2
     flushed by a 256 MB write before each, with the persistent
-    warp-specialised kernel (pipeline mode 2) and with one tile per CTA
+    warp-specialised kernel (pipeline mode 1) and with one tile per CTA
     (mode 0); the useful FLOPs and the activation bytes in and out give the
     rates."""
     import torch
@@ -637,7 +637,7 @@ def profile_conv_layers(local, batch=512, repeats=20):
             bias = torch.randn(cout, device=dev, generator=g)
             y = torch.empty(batch, p2, cout, dtype=torch.bfloat16, device=dev)
             row = {"layer": f"{cin}->{cout}", "crop": h, "batch": batch}
-            for mode in (0, 2):
+            for mode in (0, 1):
                 check(L.pfb_conv_set_pipeline(mode), "pipeline")
                 times = []
                 for it in range(3 + repeats):
@@ -820,8 +820,8 @@ def main():
     ap.add_argument("--max-steps", type=int, default=150000,
                     help="cs: plain solver steps after which a relaxation gives up")
     ap.add_argument("--conv-pipeline", type=int, default=1, choices=[0, 1, 2],
-                    help="cs: forward convolution kernel: 2 persistent warp-specialised for every "
-                         "channel pair, 1 for the 32 -> 32 pair only, 0 one tile per CTA")
+                    help="cs: forward convolution kernel: 1 (or 2, the same) persistent "
+                         "warp-specialised, 0 one tile per CTA")
     ap.add_argument("--profile-layers", action="store_true",
                     help="cs: time each U-Net layer shape's forward convolution with both kernels "
                          "and exit")

@@ -83,14 +83,14 @@ int pfb_conv3x3_wgrad(const void* x, const void* dy, float* workspace, size_t wo
 int pfb_conv3x3_wgrad_noalloc(const void* x, const void* dy, float* dw_oihw, float* db,
                               int batch, int H, int W, int cx, int cy, void* stream);
 
-/* Sticky device status of the convolution kernels: bit 0 = a wait for the
- * tensor-core MMAs gave up (the kernel skipped its output). clear != 0
- * resets it. */
+/* Sticky device status of the convolution kernels. Bit 0: a bounded wait (for
+ * a TMA copy or the tensor-core MMAs) gave up. Bit 1: a kernel found its shared
+ * memory misaligned for TMA. The forward then skips its output; the weight
+ * gradient writes NaN into its partial sums, and raises bit 0 with bit 1.
+ * clear != 0 resets it. */
 int pfb_conv_status(unsigned* out, int clear);
-/* (pfb_conv_status bit 1: the persistent forward found its shared memory
- * misaligned for TMA and computed nothing.) */
-/* Forward / data-gradient kernel choice. 1 (default) and 2: a persistent
- * warp-specialised kernel (TMA loads of the activation tiles into a two-stage
+/* Forward / data-gradient kernel choice. 1 (default; 2 is accepted as the
+ * same): a persistent warp-specialised kernel (TMA loads of the activation tiles into a two-stage
  * ring, tcgen05 MMAs into two TMEM accumulators, epilogue warps draining the
  * previous tile) where the image width allows one TMA box per half tile
  * (W <= 124); 0: one CTA per tile that stages, multiplies and writes in turn.

@@ -43,9 +43,9 @@ SOURCES = ["step2d.cu", "init2d.cu", "sim2d.cu", "host2d.cpp", "measure3d.cu", "
 CLI_SOURCES = {"pfb_cell": "cli2d.cpp", "pfb_cell_3d": "cli3d.cpp"}
 CXX = os.environ.get("CXX", "g++")
 HEADERS = ["pfb_common.cuh", "device_util.cuh", "pfb_internal.h", "step2d_common.cuh",
-           "pfb3d_common.cuh", "ring3d.cuh", "storage2d.cuh", "measure3d_common.cuh",
+           "pfb3d_common.cuh", "phi3d.cuh", "ring3d.cuh", "storage2d.cuh", "measure3d_common.cuh",
            "update3d_common.cuh",
-           "tc_util.cuh"]
+           "tc_util.cuh", "centres_csv.hpp"]
 
 
 def _newer(target: Path, deps: list[Path]) -> bool:

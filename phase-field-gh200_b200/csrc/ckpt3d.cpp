@@ -593,7 +593,8 @@ int pfb_sim3d_write_checkpoint(pfb_sim3d* s, const char* path, const pfb_ckpt3d_
     rc = pfb_sim3d_get_cells(s, cells.data());
     if (!rc) rc = pfb_sim3d_get_packed(s, phi.data());
     if (rc) return rc;
-    // the base measurement here reduces each cell over a cluster of 4 CTAs
+    // the grouping of the base measurement that the format names (the sums here
+    // are grouped by eighths of a brick, whatever the cluster size)
     return write3(path, rec, step, N, cells.data(), phi.data(), 4);
 }
 

@@ -15,10 +15,13 @@
 // Forward: out[q][co] = sum_tap sum_ci in[q + off_tap][ci] W[co][ci][tap],
 // an implicit GEMM with M = 128 positions, N = Cout, K = 9 Cin. The input
 // rows of a CTA's M-tiles plus the stencil halo are staged once in shared
-// memory as Cin/8 "chunk planes" (plane c holds channels 8c..8c+7 of every
-// staged position, 16 B per position), which is the K-major core-matrix
-// layout for every tap at once: tap (dy, dx) only moves the descriptor's
-// start row. Weights are pre-packed in global memory in the same layout.
+// memory, and one staged copy serves every tap: tap (dy, dx) only moves the
+// descriptor's start row. Two kernels: k_conv3x3_fwd_ws (persistent, warps
+// specialised; widths up to 124) stages with TMA, a position's channels in one
+// swizzled row of 64 or 32 bytes; k_conv3x3_fwd (wider images) stages with
+// cp.async as Cin/8 "chunk planes" (plane c holds channels 8c..8c+7 of every
+// staged position, 16 B per position), the K-major core-matrix layout without
+// swizzle. Weights are pre-packed in global memory in the latter layout.
 //
 // Weight gradient: dW[co][ci][tap] = sum_q dY[q][co] in[q + off_tap][ci],
 // K = positions, both operands MN-major straight from TMA; persistent CTAs
@@ -225,9 +228,12 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3_fwd(const __grid_const
 // staged once per CTA with one bulk copy. Each CTA walks tiles c, c + G,
 // c + 2G, ... of the B x tiles work list.
 //
-// Bound by the number of MMAs (45 clocks each up to N = 64, 36 a tile) and the
-// activations' DRAM traffic (143 MB, 22 us): 256 crops of 64 x 64, 32 -> 32
-// channels take 45 us (55 us gated) against 74 (84) of one tile per CTA.
+// 256 crops of 64 x 64, 32 -> 32 channels take 45 us (55 us gated) against 74
+// (84) of one tile per CTA. No unit is near its limit then: of 74 k clocks the
+// MMAs need 48 k (36 a tile, 45 clocks each at N = 32; tensor pipe 23 % active),
+// DRAM and L2 are 26 % busy, the schedulers issue on 37 % of cycles. The largest
+// stalls, long scoreboard (6.6 per issue) and short scoreboard (4.4), are of the
+// kind that the epilogue's TMEM loads and its 16-byte stores 64 bytes apart give.
 // Side-by-side taps (N = 96, a third of the MMAs, neighbouring lanes added by
 // shuffles) measured 128 us with one CTA per SM, where this form took 53.
 constexpr int kWsThreads = 64 + 128 * kConvMT;  // producer, MMA, epilogue warps of each M-tile
@@ -468,10 +474,11 @@ __global__ void __launch_bounds__(kWsThreads)
 // swizzled over that width). The 128 rows of A are 128 / CY slots of CY
 // channels, slot s the dY tile moved by s - 1 positions: one staged copy with
 // a leading offset of one row (slots past the third are not used). B holds the
-// x tiles of the three dy and a tile of ones side by side (N = 3 CX + 16: the last columns are the bias gradient),
-// so 16 positions take one MMA. The width matters: a 128-row MMA of K = 16
-// takes 45 clocks up to N = 64 and 58 at N = 112 (measured), so three of N = 32
-// or nine of one tap each would be bound by their number.
+// x tiles of the three dy and a tile of ones side by side (N = 3 CX + 16: the
+// last columns are the bias gradient), so 16 positions take one MMA. The width
+// matters: a 128-row MMA of K = 16 takes 45 clocks up to N = 48 and 58 at
+// N = 112 (measured), so three of N = 32 or nine of one tap each would be bound
+// by their number.
 //
 // Warp-specialised and persistent, one CTA per SM: CTA c owns a contiguous
 // range of the B x chunks tiles; warp 0 keeps a ring of kWgStages tiles in
@@ -481,12 +488,14 @@ __global__ void __launch_bounds__(kWsThreads)
 // towards zero, so the error of one-signed sums grows with the length of the
 // chain: 2.7e-5 of the gradient over a CTA's whole range at 256 crops of
 // 64 x 64 (457 additions), 5.6e-6 over half an image (132), 1.0e-6 over the 36
-// of a run. Two accumulators keep the MMAs going meanwhile (a layer of 256
-// crops takes 51.8 us with the reduction, 49.3 us in one chain, launches back
-// to back). 256 crops of 64 x 64, 32 -> 32
-// channels: 52 us a layer with the reduction, against about 200 of one CTA per
-// half image that staged nine shifted copies of x with cp.async; bound by the
-// TMA fill (392 rows per tile, 1.3 GB a layer through the L2).
+// of a run. Two accumulators keep the MMAs going meanwhile.
+//
+// 256 crops of 64 x 64, 32 -> 32 channels: 51.8 us a layer with the reduction,
+// launches back to back (49.3 us in one chain), against about 200 of one CTA
+// per half image that staged nine shifted copies of x with cp.async. Of the 86 k
+// clocks of a launch the MMAs need 27 k (tensor pipe 30 % active); DRAM is 38 %
+// and L2 27 % busy. What is left is the fill: 392 rows of 64 bytes a tile, 0.28
+// GB a layer, one row per 2.9 clocks and SM.
 constexpr int kWgStages = 6;
 constexpr int kWgThreads = 192;
 constexpr int kWgKT = 96;        // positions per tile: divides 64 x 66 exactly
@@ -799,8 +808,8 @@ cudaError_t launch_fwd(const ConvFwdArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// 0: one tile per CTA; 1 and 2: the persistent warp-specialised forward for
-// every built pair where two TMA boxes hold a tile's rows (W <= 124).
+// 0: one tile per CTA; 1 (2 is accepted as the same): the persistent
+// warp-specialised forward where two TMA boxes hold a tile's rows (W <= 124).
 int g_conv_pipeline = 1;
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {

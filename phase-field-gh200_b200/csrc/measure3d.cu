@@ -1,14 +1,14 @@
 // 3D measurement and motion (sm_100a).
 //
-// k_measure3d<K>: one thread-block cluster of K CTAs per cell (K as in the
-// fused step k_step3d for the same brick edge, so both group the FP64 sums
-// alike); CTA r walks
-// brick planes [r B/K, (r+1) B/K) through a ring of bulk-copied planes and
+// k_measure3d<K>: one thread-block cluster of K CTAs per cell, 4 or 8; CTA r
+// walks brick planes [r B/K, (r+1) B/K) through a ring of bulk-copied planes and
 // accumulates V, the centroid sums, the interaction integral, the surface
-// proxy, the support box and phi_max of its planes. The K partial results
-// are pushed into rank 0's shared memory with st.async and summed there in
-// rank order; rank 0 then plans the recentring shift and checks the support
-// margin exactly as the reference's commit_measurement
+// proxy, the support box and phi_max of its planes. The sums are kept per
+// eighth of the brick whatever K (and in the fused step k_step3d), so that all
+// give the same bits. The eight partial records are pushed into rank 0's shared
+// memory with st.async and summed there in plane order; rank 0 then plans the
+// recentring shift and checks the support margin exactly as the reference's
+// commit_measurement
 // (src/pf3d/kernels.cu:418-497). Per-voxel semantics follow
 // measure_one_cell (src/pf3d/kernels.cu:1271-1409).
 //

@@ -11,7 +11,7 @@
 //   phase A  measures its planes (the same per-voxel sums and grouping as
 //            k_measure3d),
 //   fold     pushes its partial record into rank 0 with st.async; rank 0
-//            folds the 4 records in rank order, commits the measured record
+//            folds the eight records in plane order, commits the measured record
 //            and the recentring plan, applies the tumble and velocity, and
 //            pushes {V, velocity, shift, keep} back into every rank. While
 //            the fold runs, each CTA already restages the first planes of

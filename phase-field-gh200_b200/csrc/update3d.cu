@@ -6,15 +6,15 @@
 // 54-318) and k_update_tiled_fast (src/pf3d/kernels.cu:498-793) on the same
 // inputs, and every sticky flag is raised as often as there.
 //
-// Layout of the work: K CTAs per cell, CTA r owns destination planes
-// [r B/K, (r+1) B/K). Destination plane dz reads source plane dz + sz and
-// its two neighbours from a ring of whole brick planes staged by bulk
-// copies (one 16 KB copy per plane at B = 64). A thread owns a strip of 4
-// voxels x 4 rows and walks the rows with a three-row register window per
-// source plane; the aggregate S_in is read from L2 one row ahead; phi_out is
-// written with 16-byte streaming stores (every destination voxel once, so the
-// output needs no clearing pass) and S_out receives one predicated atomic per
-// non-zero voxel.
+// Layout of the work: 4 CTAs per cell, up to B/2 where a system has few cells;
+// CTA r of P owns destination planes [r B/P, (r+1) B/P). Destination plane dz
+// reads source plane dz + sz and its two neighbours from a ring of whole brick
+// planes staged by bulk copies (one 16 KB copy per plane at B = 64). A thread
+// owns a strip of 4 voxels x 4 rows and walks the rows with a three-row register
+// window per source plane; the aggregate S_in is read from L2 one row ahead;
+// phi_out is written with 16-byte streaming stores (every destination voxel
+// once, so the output needs no clearing pass) and S_out receives one predicated
+// atomic per non-zero voxel.
 #include <cuda_runtime.h>
 
 #include <vector>

@@ -1,6 +1,6 @@
 """The driver's default scatter (variants 0/1): the identity path adds q(phi)
 into the Q5.27 aggregate with non-returning red.add, and S_overflow stays
-exact through per-bin bounds recounted by the launch's last CTA. Checked on a
+exact through per-bin bounds settled by the next launch or when the advance ends. Checked on a
 B200 against the returning scatter (variant 2) and against the reference's own
 kernel (oracle/_ref/libref2d.so), which tests the value returned by every add
 (src/kernels.cu:496-497):
