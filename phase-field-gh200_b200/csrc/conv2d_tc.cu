@@ -487,21 +487,21 @@ __global__ void __launch_bounds__(kWsThreads)
 // those at the end. The tensor core adds into its accumulator with a bias
 // towards zero, so the error of one-signed sums grows with the length of the
 // chain: 2.7e-5 of the gradient over a CTA's whole range at 256 crops of
-// 64 x 64 (457 additions), 5.6e-6 over half an image (132), 1.0e-6 over the 36
+// 64 x 64 (457 additions), 5.6e-6 over half an image (132), 2.2e-6 over the 66
 // of a run. Two accumulators keep the MMAs going meanwhile.
 //
-// 256 crops of 64 x 64, 32 -> 32 channels: 51.8 us a layer with the reduction,
-// launches back to back (49.3 us in one chain), against about 200 of one CTA
-// per half image that staged nine shifted copies of x with cp.async. Of the 86 k
-// clocks of a launch the MMAs need 27 k (tensor pipe 30 % active); DRAM is 38 %
-// and L2 27 % busy. What is left is the fill: 392 rows of 64 bytes a tile, 0.28
+// 256 crops of 64 x 64, 32 -> 32 channels: 50.1 us a layer with the reduction,
+// launches back to back (49.5 us with runs of half an image, 51.2 of 6 tiles),
+// against about 200 of one CTA per half image that staged nine shifted copies of
+// x with cp.async. Of the 86 k clocks of a launch the MMAs need 27 k (tensor
+// pipe 30 % active); DRAM is 38 % and L2 27 % busy. What is left is the fill: 392 rows of 64 bytes a tile, 0.28
 // GB a layer, one row per 2.9 clocks and SM.
 constexpr int kWgStages = 6;
 constexpr int kWgThreads = 192;
 constexpr int kWgKT = 96;        // positions per tile: divides 64 x 66 exactly
 constexpr int kWgHeader = 1024;  // barriers
 constexpr uint32_t kWgCols = 128;  // TMEM columns of an accumulator: CX per dy, then 16 of the bias
-constexpr int kWgRun = 6;        // most tiles summed in one accumulator
+constexpr int kWgRun = 11;       // most tiles summed in one accumulator
 
 constexpr int kWgYRows = kWgKT + 8;  // dY rows staged: the last slot is moved by 7 at most
 // A stage: the dY tile, three x tiles, a tile of ones.
@@ -692,20 +692,11 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             // NaN instead of mixing in what the scratch held before
             for (int i = tid - 64; i < 9 * CY * CX + CY; i += 128) out[i] = __int_as_float(0x7fc00000);
         } else if (slot < 3) {
-            const bool vec = (reinterpret_cast<uintptr_t>(A.partial) & 15u) == 0u;
+            // the lanes' output channels side by side
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                float* o = out + ((3 * d + 2 - slot) * CY + co) * CX;
-                if (vec) {
+            for (int d = 0; d < 3; ++d)
 #pragma unroll
-                    for (int j = 0; j < CX; j += 4)
-                        *reinterpret_cast<float4*>(o + j) = make_float4(sum[d * CX + j], sum[d * CX + j + 1],
-                                                                        sum[d * CX + j + 2], sum[d * CX + j + 3]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < CX; ++j) o[j] = sum[d * CX + j];
-                }
-            }
+                for (int j = 0; j < CX; ++j) out[((3 * d + 2 - slot) * CX + j) * CY + co] = sum[d * CX + j];
             if (slot == 1) out[9 * CY * CX + co] = bias;
         }
     }
@@ -714,7 +705,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     if (warp == 0) tc::tmem_dealloc(tmem, 2 * kWgCols);
 }
 
-// dW[co][ci][tap] = sum over CTAs of partial[cta][tap][co][ci]; db[co] likewise.
+// dW[co][ci][tap] = sum over CTAs of partial[cta][tap][ci][co]; db[co] likewise.
 // Two levels in a fixed order: thread row j of a CTA sums the blocks
 // g = j, j + 16, j + 32, ... of 32 consecutive outputs (each warp reads 128
 // contiguous bytes per block), then the 16 row sums are added in row order.
@@ -749,7 +740,7 @@ __global__ void __launch_bounds__(kRedCols * kRedRows)
     for (int r = 1; r < kRedRows; ++r) t += part[r][threadIdx.x];
     if (i < 9 * cy * cx) {
         const int tap = i / (cy * cx), rem = i - tap * cy * cx;
-        const int co = rem / cx, ci = rem - co * cx;
+        const int ci = rem / cy, co = rem - ci * cy;
         dw[((size_t)co * cx + ci) * 9 + tap] = t;
     } else if (db) {
         db[i - 9 * cy * cx] = t;

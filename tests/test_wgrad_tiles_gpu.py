@@ -9,10 +9,10 @@ terms plus 1e-5, as for the other weight-gradient tests.
 
 The tensor core's binary32 accumulator rounds towards zero, so a sum of one sign
 falls short by up to 2^-23 of its running value with every addition: half a
-chain's length times 2^-23 of the total. A chain is 36 additions (6 tiles) at
-most, 2.1e-6; adding up the chains (13 per CTA and 25 in the reduction, to
-nearest, 2^-24 each of a running sum) gives up to 1.2e-6. The last test asks
-for 4e-6 however many images a CTA walks."""
+chain's length times 2^-23 of the total. A chain is 66 additions (11 tiles) at
+most, 3.9e-6; adding up the chains (7 per CTA and 25 in the reduction, to
+nearest, 2^-24 each of a running sum) gives up to 1.0e-6. The last test asks
+for 5e-6 however many images a CTA walks."""
 import ctypes as C
 
 import numpy as np
@@ -76,5 +76,5 @@ def test_error_does_not_grow_with_the_batch(cx, cy, B, H, W):
     torch.cuda.synchronize()
     rdw, rdb = co.conv3x3_wgrad(co.from_padded(xd.float().cpu().numpy(), H, W),
                                 co.from_padded(yd.float().cpu().numpy(), H, W))
-    assert np.max(np.abs(dw.cpu().numpy() / rdw - 1.0)) <= 4e-6
-    assert np.max(np.abs(db.cpu().numpy() / rdb - 1.0)) <= 4e-6
+    assert np.max(np.abs(dw.cpu().numpy() / rdw - 1.0)) <= 5e-6
+    assert np.max(np.abs(db.cpu().numpy() / rdb - 1.0)) <= 5e-6
